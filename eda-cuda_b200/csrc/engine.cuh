@@ -381,8 +381,23 @@ enum class CubeOp : int8_t { kMax = 0, kMin = 1, kMaxMin = 2, kBox = 3 };
 // bit field (src_bits: bit `bit` of a u8 field, as 0 / 1); the last pass of a box cube may apply
 // an epilogue instead of a plain store.
 enum class BoxEpi : int8_t {
-  kStore = 0,   // out = box
-  kDetSq = 1,   // out = (aux - box)^2 (the detail energy of the threshold field; aux = r)
+  kStore = 0,  // out = box
+  kDetSq = 1,  // out = (aux - box)^2 (the detail energy of the threshold field; aux = r)
+  kTau = 2,    // out = the threshold of the detail energy's box (tau_field)
+  kRho = 3,    // out = aux + box^2 (aux nullptr: box^2), `finish`: the raw window of that sum (raw_window)
+  kClip = 4,   // out = box clipped to [0, 1]
+  kExp = 5,    // out = exp(box)
+};
+template <class T>
+struct BoxEpilogue {
+  BoxEpi kind;
+  const T* aux;            // the second operand, at the output's place
+  T* out;                  // where the last pass writes (nullptr: the cube's out0)
+  const int32_t* run;      // [B] elements to filter (nullptr: those with a window)
+  Elem* el;                // kTau: sigma_n, sigma_x, tol; nonfinite is set
+  double sig_noise, sig_theta, fine_theta;
+  int32_t floor2, finish;
+  T two_kappa, tiny;       // kRho
 };
 template <class T>
 struct CubeArgs {
@@ -394,29 +409,32 @@ struct CubeArgs {
   const int32_t* win;         // [rungs * B] odd windows (< 1: skip the element)
   int32_t rungs;              // > 1: rung j reads win + j B and writes out + j * out_stride
   int64_t out_stride;
-  BoxEpi epi;
-  const T* aux;
+  BoxEpilogue<T> epi;         // box only
 };
 template <class T>
 void cube(cudaStream_t s, const Geom& g, CubeOp op, const CubeArgs<T>& a);
 template <class T>
 void cube_simple(cudaStream_t s, const Geom& g, CubeOp op, const T* in, T* out0, T* out1, const int32_t* win);
-// The launch shape of a cube pass: lines per CTA (1, 2, 4 or 8), line groups per CTA, and the
-// segment share from which a window folds whole segments per worker; 0 leaves the default. The
-// shapes change no bit of any result (the folds are canonical): tune.cu times them per geometry
-// and keeps the fastest (eda_autotune); cube_tune_for returns the recorded shape of a pass, or the
-// calling thread's override while tuning.
+// The launch shape of a cube pass: lines per CTA (1, 2, 4 or 8); 0 leaves the default (groups and
+// seq_share belong to the cache file's format only). The shapes change no bit of any result: tune.cu
+// times them per geometry and keeps the fastest (eda_autotune); cube_tune_for returns the recorded
+// shape of a pass, or the calling thread's override while tuning.
 struct CubeTune {
   int32_t lines = 0, groups = 0, seq_share = 0;
 };
 CubeTune cube_tune_for(const Geom& g, int axis, size_t es);
 void cube_tune_override(const CubeTune* t);  // nullptr: none (per calling thread)
 
-// 1-D lines too long for a pass to stage in shared memory fold in global memory: the calling host
-// thread provides a scratch of long_line_scratch_bytes (batch x pitch samples; 0 when the lines
-// fit) for the lines' fold input, before its cube calls.
+// 1-D lines too long for a pass to stage whole are cut into tiles: the calling host thread provides
+// two scratch buffers before its cube calls, of long_line_scratch_bytes (the lines' samples and their
+// blocks' extremes) and long_totals_scratch_bytes (the chunk totals of the box passes, free between
+// them); both 0 when the lines are staged.
 size_t long_line_scratch_bytes(const Geom& g, size_t es);
-void set_long_line_scratch(void* p, size_t bytes);
+size_t long_totals_scratch_bytes(const Geom& g, size_t es);
+void set_long_line_scratch(void* lines, void* totals);
+// What a call with 1-D lines of more than a CTA's shared memory (18 900 float32 samples) is accounted
+// for besides the engine's fields (engine_bytes).
+size_t fold_scratch_bytes(const Geom& g, size_t es);
 
 // Canonical reductions: per element sum v^2 (canonical tree) and max|v| of f.
 template <class T>

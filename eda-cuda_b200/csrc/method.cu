@@ -669,8 +669,8 @@ void Engine<T>::tau_field(const int32_t* run, bool floor2, T* tau) {
   a.out0 = tmp_;
   a.win = win(kWd);
   a.rungs = 1;
-  a.epi = BoxEpi::kDetSq;
-  a.aux = r_;
+  a.epi.kind = BoxEpi::kDetSq;
+  a.epi.aux = r_;
   cube<T>(s_, g_, CubeOp::kBox, a);
   cube_simple<T>(s_, g_, CubeOp::kBox, tmp_, tau, nullptr, win(kWl));
   const Ctl c = c_;
@@ -1638,16 +1638,16 @@ size_t engine_bytes(const Geom& g) {
   if (D >= 2) b += static_cast<size_t>(orient_work_samples(g)) * sizeof(T);
   b += static_cast<size_t>(g.batch) * (sizeof(Elem) + 4 * (kSlots + kMasks + kMaxRungs) + 8 * 10 + 64);
   b += select_scratch_bytes(g) + totals_scratch_bytes(g);
-  b += long_line_scratch_bytes(g, sizeof(T));  // 1-D lines beyond the cube passes' staged capacity
+  b += fold_scratch_bytes(g, sizeof(T)) + long_line_scratch_bytes(g, sizeof(T));
   b += 160 * 256;  // every take is rounded up to 256 bytes
   return b;
 }
 
 namespace {
-// The long-line scratch of the calling thread for the duration of one engine run.
+// The long lines' scratch of the calling thread for the duration of one engine run.
 struct LongLineScratch {
-  LongLineScratch(void* p, size_t bytes) { set_long_line_scratch(p, bytes); }
-  ~LongLineScratch() { set_long_line_scratch(nullptr, 0); }
+  LongLineScratch(void* lines, void* totals) { set_long_line_scratch(lines, totals); }
+  ~LongLineScratch() { set_long_line_scratch(nullptr, nullptr); }
 };
 }  // namespace
 
@@ -1657,7 +1657,9 @@ void run_chunk(const Geom& g, const Ctl& c, cudaStream_t s, Workspace& ws, const
   Engine<T> e(g, c, s, ws);
   e.orient_out_ = g.dim >= 2 ? orient : nullptr;
   const size_t lb = long_line_scratch_bytes(g, sizeof(T));
-  const LongLineScratch scratch(lb ? ws.take<unsigned char>(lb) : nullptr, lb);
+  const size_t rung_bytes = static_cast<size_t>(g.batch * g.field) * kMaxRungs * sizeof(T);
+  if (long_totals_scratch_bytes(g, sizeof(T)) > rung_bytes) throw std::logic_error("edab: long-line totals exceed the rungs");
+  const LongLineScratch scratch(lb ? ws.take<unsigned char>(lb) : nullptr, lb ? e.rung1_ : nullptr);
   e.run(x, rows, hs, hf, hp, he, out);
 }
 

@@ -60,11 +60,11 @@ void run_cube(const void* x_dev, int dim, int64_t batch, const int64_t* n, int o
   const unsigned blocks = blocks_for(fe);
   to_padded<T><<<std::min(blocks, 1u << 16), kThreads, 0, s>>>(g, static_cast<const T*>(x_dev), in);
   EDAB_LAUNCH("to_padded");
-  // 1-D lines beyond the staged capacity fold through a global scratch of batch x pitch samples
+  // 1-D lines that are not staged whole go through a global scratch
   const size_t lb = long_line_scratch_bytes(g, sizeof(T));
   void* ls = nullptr;
-  if (lb) EDAB_CUDA(cudaMalloc(&ls, lb));
-  set_long_line_scratch(ls, lb);
+  if (lb) EDAB_CUDA(cudaMalloc(&ls, lb + long_totals_scratch_bytes(g, sizeof(T))));
+  set_long_line_scratch(ls, lb ? static_cast<char*>(ls) + lb : nullptr);
   CubeArgs<T> a{};
   a.in = in;
   a.out0 = o0;
@@ -72,7 +72,6 @@ void run_cube(const void* x_dev, int dim, int64_t batch, const int64_t* n, int o
   a.win = dw;
   a.rungs = rungs;
   a.out_stride = fe;
-  a.epi = BoxEpi::kStore;
   cube<T>(s, g, static_cast<CubeOp>(op), a);
   const unsigned ob = blocks_for(batch * rungs * g.count);
   to_dense<T><<<std::min(ob, 1u << 16), kThreads, 0, s>>>(g, batch * rungs, o0, static_cast<T*>(out0));
@@ -82,7 +81,7 @@ void run_cube(const void* x_dev, int dim, int64_t batch, const int64_t* n, int o
     EDAB_LAUNCH("to_dense");
   }
   EDAB_CUDA(cudaStreamSynchronize(s));
-  set_long_line_scratch(nullptr, 0);
+  set_long_line_scratch(nullptr, nullptr);
   cudaFree(ls);
   cudaFree(in);
   cudaFree(o0);

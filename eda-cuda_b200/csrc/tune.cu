@@ -1,9 +1,10 @@
 // SPDX-License-Identifier: Apache-2.0
 // The cube passes' autotuner (no counterpart in the reference, whose launch shapes are fixed:
-// vhgw_lines_per_cta, cpp/src/field/vhgw.cu:540-559). A pass's launch shape (lines per CTA, line
-// groups per CTA, the segment share from which windows fold whole segments) changes no bit of any
-// result, only its speed, and the best shape depends on the geometry: the axis lengths (line and
-// segment counts per CTA), the batch (waves of CTAs) and the dtype. eda_autotune times every
+// vhgw_lines_per_cta, cpp/src/field/vhgw.cu:540-559). A pass's launch shape (lines per CTA) changes
+// no bit of any result, only its speed, and the best shape depends on the geometry: the axis lengths,
+// the batch (waves of CTAs) and the dtype. (A record also holds the line groups per CTA and the
+// segment share of earlier passes, which the cache file's format keeps and no pass reads: the groups
+// follow from the launch, and every window folds by chunks.) eda_autotune times every
 // candidate shape on a synthetic field of the geometry, through a max+min and a box cube over a
 // ladder of windows like the method's, and records the fastest for that geometry; the records
 // live in a table of the process, can be saved to and loaded from a text file (the on-disk
@@ -125,6 +126,7 @@ TuneRecord tune_geometry(const Geom& g, cudaStream_t s) {
   const int32_t R = static_cast<int32_t>(wins.size());
   const int64_t fe = g.batch * g.field;
   T *in = nullptr, *o0 = nullptr, *o1 = nullptr;
+  void* lines = nullptr;  // the scratch of long 1-D lines
   int32_t* dw = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   std::vector<int32_t> hw(static_cast<size_t>(R) * g.batch);
@@ -136,6 +138,10 @@ TuneRecord tune_geometry(const Geom& g, cudaStream_t s) {
     EDAB_CUDA(cudaMalloc(&o0, fe * R * sizeof(T)));
     EDAB_CUDA(cudaMalloc(&o1, fe * R * sizeof(T)));
     EDAB_CUDA(cudaMalloc(&dw, hw.size() * sizeof(int32_t)));
+    if (const size_t lb = long_line_scratch_bytes(g, sizeof(T))) {
+      EDAB_CUDA(cudaMalloc(&lines, lb + long_totals_scratch_bytes(g, sizeof(T))));
+      set_long_line_scratch(lines, static_cast<char*>(lines) + lb);
+    }
     EDAB_CUDA(cudaMemcpyAsync(dw, hw.data(), hw.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
     fill_noise<T><<<blocks_for(std::min<int64_t>(fe, 1 << 24)), kThreads, 0, s>>>(in, fe, 12345);
     EDAB_LAUNCH("fill_noise");
@@ -153,7 +159,6 @@ TuneRecord tune_geometry(const Geom& g, cudaStream_t s) {
         a.win = dw;
         a.rungs = R;
         a.out_stride = fe;
-        a.epi = BoxEpi::kStore;
         cube<T>(s, g, CubeOp::kMaxMin, a);
         a.out1 = nullptr;
         cube<T>(s, g, CubeOp::kBox, a);
@@ -169,19 +174,17 @@ TuneRecord tune_geometry(const Geom& g, cudaStream_t s) {
     best.us_default = time_shape(nullptr);
     best.us_best = best.us_default;
     for (int lines : {8, 4, 2}) {
-      for (int groups : {1, 2}) {
-        for (int share : {2, 4, 8}) {
-          const CubeTune t{lines, groups, share};
-          const double us = time_shape(&t);
-          if (us < best.us_best) {
-            best.us_best = us;
-            best.tune = t;
-          }
-        }
+      const CubeTune t{lines, 0, 0};
+      const double us = time_shape(&t);
+      if (us < best.us_best) {
+        best.us_best = us;
+        best.tune = t;
       }
     }
   } catch (...) {
     cube_tune_override(nullptr);
+    set_long_line_scratch(nullptr, nullptr);
+    cudaFree(lines);
     cudaFree(in);
     cudaFree(o0);
     cudaFree(o1);
@@ -190,6 +193,8 @@ TuneRecord tune_geometry(const Geom& g, cudaStream_t s) {
     if (e1) cudaEventDestroy(e1);
     throw;
   }
+  set_long_line_scratch(nullptr, nullptr);
+  cudaFree(lines);
   cudaFree(in);
   cudaFree(o0);
   cudaFree(o1);
