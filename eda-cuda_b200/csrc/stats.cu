@@ -832,13 +832,94 @@ __device__ bool side_falls(const X& x, int32_t n, int32_t p, T v, T tau, const T
   return false;
 }
 
+// The run of samples equal to x(s) from s, when s starts one (x(s - 1) differs): its middle sample as
+// the peak pk, and 1 for a maximum, 2 for a minimum, 0 for neither.
+template <class T, class X>
+__device__ __forceinline__ int peak_at(const X& x, int32_t n, int32_t nb, int32_t s, const T* bmin, const T* bmax,
+                                       int32_t* pk) {
+  const T cur = x(s), prev = x(s - 1);
+  if (!(prev < cur || prev > cur)) return 0;
+  int32_t e;
+  const int32_t lim = min((s / kBlk) * kBlk + kBlk - 1, n - 1);
+  int32_t k = s + 1;
+  while (k <= lim && x(k) == cur) ++k;
+  if (k <= lim || k >= n) {
+    e = k - 1;
+  } else {
+    e = n - 1;
+    for (int32_t c = k / kBlk; c < nb; ++c) {
+      if (bmin[c] == cur && bmax[c] == cur) continue;
+      k = c * kBlk;
+      while (x(k) == cur) ++k;
+      e = k - 1;
+      break;
+    }
+  }
+  if (e > n - 2) return 0;
+  const T nxt = x(e + 1);
+  *pk = (s + e) / 2;
+  return prev < cur && nxt < cur ? 1 : (prev > cur && nxt > cur ? 2 : 0);
+}
+
+// Whether the peak pk (kind 1: maximum, 2: minimum) falls by tau on both sides.
+template <class T, class X>
+__device__ __forceinline__ bool peak_counts(const X& x, int32_t n, int32_t pk, int kind, T tau, const T* bmin,
+                                            const T* bmax) {
+  const T v = x(pk);
+  return kind == 1 ? side_falls<true, -1>(x, n, pk, v, tau, bmax, bmin) && side_falls<true, 1>(x, n, pk, v, tau, bmax, bmin)
+                   : side_falls<false, -1>(x, n, pk, v, tau, bmin, bmax) && side_falls<false, 1>(x, n, pk, v, tau, bmin, bmax);
+}
+
+// A warp's peaks waiting to be judged. Testing a sample for a peak is short and the same for every
+// lane; walking a peak's sides is long, and only a third of the samples of a noisy line are peaks.
+// So the lanes that find peaks push them here, and the warp judges 32 at a time, every lane one.
+constexpr int kPeakQueue = 64;
+template <class Judge>
+__device__ __forceinline__ void push_peaks(uint32_t* queue, int& held, bool found, uint32_t entry, const Judge& judge) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = __ballot_sync(0xffffffffu, found);
+  if (found) queue[held + __popc(m & ((1u << lane) - 1u))] = entry;
+  held += __popc(m);
+  __syncwarp();
+  if (held >= 32) {
+    held -= 32;
+    judge(queue[held + lane]);
+    __syncwarp();
+  }
+}
+template <class Judge>
+__device__ __forceinline__ void drain_peaks(const uint32_t* queue, int held, const Judge& judge) {
+  if (static_cast<int>(threadIdx.x & 31) < held) judge(queue[threadIdx.x & 31]);
+}
+
+__device__ __forceinline__ void copy_async(float* smem, const float* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem))),
+               "l"(gmem)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async(double* smem, const double* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem))),
+               "l"(gmem)
+               : "memory");
+}
+
+// The inner samples [first, end) of a line of n that part blockIdx.x % parts of it takes.
+__device__ __forceinline__ void part_of_line(int32_t n, int32_t* first, int32_t* end, int32_t parts, int32_t part) {
+  const int32_t per = ((n - 2 + parts - 1) / parts + 31) & ~31;
+  *first = 1 + part * per;
+  *end = min(*first + per, n - 1);
+}
+
 // Staged lines: P lines of LX words (sample k at k + k / 32; LX odd, so lanes on consecutive lines
-// hit distinct banks), then the block minima and maxima. Rows: threads over the samples of a line;
-// column panels: lanes over the panel's columns (coalesced tau reads and flag writes).
+// hit distinct banks), then the block minima and maxima. Rows: a warp takes 32 consecutive samples of
+// a line; column panels: its lanes cover the panel's columns (whole sectors of flags and tau). What
+// bounds it: the walks of the peaks' sides (shared-memory latency, lanes with walks of different
+// lengths); staging is asynchronous, all of a thread's samples in flight at once.
 template <class T>
 __global__ void __launch_bounds__(kThreads) flags_pass(Geom g, int axis, const T* __restrict__ r,
                                                        const T* __restrict__ tau, uint8_t* __restrict__ flags,
-                                                       Elem* el, const int32_t* run, int P, int32_t LX) {
+                                                       Elem* el, const int32_t* run, int P, int32_t LX,
+                                                       int32_t parts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t b = blockIdx.y;
   if (run && !run[b]) return;
@@ -851,7 +932,13 @@ __global__ void __launch_bounds__(kThreads) flags_pass(Geom g, int axis, const T
   __shared__ int64_t base_s[64];
   __shared__ int32_t ok_s[64];
   __shared__ int32_t count_s;
-  const int64_t grp = blockIdx.x;
+  __shared__ uint32_t queue_s[kThreads / 32][kPeakQueue];
+  const int64_t grp = parts > 1 ? blockIdx.x / parts : blockIdx.x;
+  int32_t s_first = 1, s_end = n - 1;
+  if (parts > 1) {
+    part_of_line(n, &s_first, &s_end, parts, static_cast<int32_t>(blockIdx.x % parts));
+    if (s_first >= s_end) return;
+  }
   if (threadIdx.x < P) {
     const int p = threadIdx.x;
     bool ok;
@@ -861,12 +948,13 @@ __global__ void __launch_bounds__(kThreads) flags_pass(Geom g, int axis, const T
       ok = row < g.rows;
       base = row * g.pitch;
     } else {
-      const int64_t inner = geom_stride(g, axis);
-      const int64_t gpo = (inner + P - 1) / P;
-      const int64_t o = grp / gpo;
-      const int64_t c = (grp - o * gpo) * P + p;
-      ok = c < inner && (c % g.pitch) < g.n_last;
-      base = o * static_cast<int64_t>(n) * inner + c;
+      // 32-bit divisions (an element holds fewer than 2^31 samples)
+      const uint32_t inner = static_cast<uint32_t>(geom_stride(g, axis));
+      const uint32_t gpo = (inner + P - 1) / P;
+      const uint32_t o = static_cast<uint32_t>(grp) / gpo;
+      const uint32_t c = (static_cast<uint32_t>(grp) - o * gpo) * P + p;
+      ok = c < inner && static_cast<int32_t>(c % static_cast<uint32_t>(g.pitch)) < g.n_last;
+      base = static_cast<int64_t>(o) * n * inner + c;
     }
     base_s[p] = base;
     ok_s[p] = ok ? 1 : 0;
@@ -874,14 +962,17 @@ __global__ void __launch_bounds__(kThreads) flags_pass(Geom g, int axis, const T
   if (threadIdx.x == 0) count_s = 0;
   const int64_t step = contig ? 1 : geom_stride(g, axis);
   const int64_t eoff = b * g.field;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __syncthreads();
   if (contig) {
-    // lines in turn, consecutive samples over the threads
-    for (int p = 0; p < P; ++p) {
+    // a warp stages 1 / share of a line
+    const int share = P >= kThreads / 32 ? 1 : kThreads / 32 / P;
+    for (int q = warp; q < P * share; q += kThreads / 32) {
+      const int p = q / share;
       if (!ok_s[p]) continue;
       const T* src = r + eoff + base_s[p];
       T* x = X + p * LX;
-      for (int32_t i = threadIdx.x; i < n; i += blockDim.x) x[i + (i >> 5)] = src[i];
+      for (int32_t i = lane + 32 * (q - p * share); i < n; i += 32 * share) copy_async(x + i + (i >> 5), src + i);
     }
   } else {
     // the P columns of a row over consecutive threads (whole sectors); one division per thread
@@ -891,9 +982,10 @@ __global__ void __launch_bounds__(kThreads) flags_pass(Geom g, int axis, const T
     if (i0 < rows_per && ok_s[p]) {
       const T* src = r + eoff + base_s[p];
       T* x = X + p * LX;
-      for (int32_t i = i0; i < n; i += rows_per) x[i + (i >> 5)] = src[static_cast<int64_t>(i) * step];
+      for (int32_t i = i0; i < n; i += rows_per) copy_async(x + i + (i >> 5), src + static_cast<int64_t>(i) * step);
     }
   }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
   for (int32_t t = threadIdx.x; t < P * nb; t += blockDim.x) {
     const int p = t / nb;
@@ -911,143 +1003,118 @@ __global__ void __launch_bounds__(kThreads) flags_pass(Geom g, int axis, const T
     bmax[p * nb + c] = mx;
   }
   __syncthreads();
-  int mine = 0;
-  // the run of samples equal to x[s] from s (s a run start): significant extremum -> flag its peak
-  const auto visit = [&](int p, int32_t s) {
-    const T* x = X + p * LX;
-    // the threshold at s, read for every sample (coalesced over the warp) ahead of its use at a peak
-    const T tp_s = tau[eoff + base_s[p] + s * step];
-    const T cur = xs(x, s), prev = xs(x, s - 1);
-    if (!(prev < cur || prev > cur)) return;
-    const T* pmin = bmin + p * nb;
-    const T* pmax = bmax + p * nb;
-    int32_t e;
-    {
-      const int32_t lim = min((s / kBlk) * kBlk + kBlk - 1, n - 1);
-      int32_t k = s + 1;
-      while (k <= lim && xs(x, k) == cur) ++k;
-      if (k <= lim || k >= n) {
-        e = k - 1;
-      } else {
-        e = n - 1;
-        for (int32_t c = k / kBlk; c < nb; ++c) {
-          if (pmin[c] == cur && pmax[c] == cur) continue;
-          k = c * kBlk;
-          while (xs(x, k) == cur) ++k;
-          e = k - 1;
-          break;
-        }
-      }
-    }
-    if (e > n - 2) return;
-    const T nxt = xs(x, e + 1);
-    const bool is_max = prev < cur && nxt < cur;
-    const bool is_min = prev > cur && nxt > cur;
-    if (!is_max && !is_min) return;
-    const int32_t pk = (s + e) / 2;
+  int mine = 0, held = 0;
+  uint32_t* queue = queue_s[warp];
+  // a queued peak: its sample (below 2^24), line (6 bits) and kind
+  const auto judge = [&](uint32_t entry) {
+    const int32_t pk = static_cast<int32_t>(entry & 0xffffffu);
+    const int p = static_cast<int>(entry >> 24) & 63;
     const int64_t at = eoff + base_s[p] + pk * step;
-    const T tp = pk == s ? tp_s : tau[at];
+    const T tp = tau[at];
+    const T* x = X + p * LX;
     const auto at_k = [x](int32_t k) { return xs(x, k); };
-    const bool sig = is_max ? side_falls<true, -1>(at_k, n, pk, cur, tp, pmax, pmin) && side_falls<true, 1>(at_k, n, pk, cur, tp, pmax, pmin)
-                            : side_falls<false, -1>(at_k, n, pk, cur, tp, pmin, pmax) && side_falls<false, 1>(at_k, n, pk, cur, tp, pmin, pmax);
-    if (sig) {
+    if (peak_counts<T>(at_k, n, pk, static_cast<int>(entry >> 30), tp, bmin + p * nb, bmax + p * nb)) {
       flags[at] |= static_cast<uint8_t>(1u << axis);
       ++mine;
     }
   };
+  // the warp's lanes together: lane's sample s of line p (valid: inside the line)
+  const auto visit = [&](int p, int32_t s, bool valid) {
+    int kind = 0;
+    int32_t pk = 0;
+    if (valid) {
+      const T* x = X + p * LX;
+      const auto at_k = [x](int32_t k) { return xs(x, k); };
+      kind = peak_at<T>(at_k, n, nb, s, bmin + p * nb, bmax + p * nb, &pk);
+    }
+    push_peaks(queue, held, kind != 0,
+               static_cast<uint32_t>(pk) | static_cast<uint32_t>(p) << 24 | static_cast<uint32_t>(kind) << 30, judge);
+  };
   if (contig) {
-    for (int p = 0; p < P; ++p) {
+    const int32_t runs = (s_end - s_first + 31) / 32;  // 32-sample runs of a line's inner samples
+    for (int32_t q = warp; q < P * runs; q += kThreads / 32) {
+      const int p = q / runs;
       if (!ok_s[p]) continue;
-      for (int32_t s = 1 + threadIdx.x; s <= n - 2; s += blockDim.x) visit(p, s);
+      const int32_t s = s_first + 32 * (q - p * runs) + lane;
+      visit(p, s, s < s_end);
     }
   } else {
     // lanes over the panel's columns; a warp covers 32 / P rows (P a power of two <= 32)
     const int p = threadIdx.x & (P - 1);
     const int32_t rpw = 32 / P;
     const int32_t nrows = static_cast<int32_t>(blockDim.x >> 5) * rpw;
-    if (ok_s[p]) {
-      for (int32_t s = 1 + static_cast<int32_t>(threadIdx.x / P); s <= n - 2; s += nrows) visit(p, s);
+    const bool ok = ok_s[p] != 0;
+    for (int32_t s0 = 1 + warp * rpw; s0 <= n - 2; s0 += nrows) {
+      const int32_t s = s0 + lane / P;
+      visit(p, s, ok && s <= n - 2);
     }
   }
+  drain_peaks(queue, held, judge);
   for (int d = 16; d > 0; d >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, d);
-  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&count_s, mine);
+  if (lane == 0 && mine) atomicAdd(&count_s, mine);
   __syncthreads();
   if (threadIdx.x == 0 && count_s) {
     atomicAdd(reinterpret_cast<unsigned long long*>(&el[b].ext[axis]), static_cast<unsigned long long>(count_s));
   }
 }
 
-// Lines too long to stage (1-D signals beyond the staged capacity): one CTA per line reads the
-// samples from global memory (L1 / L2) and keeps only the 32-sample block extremes in shared
-// memory; the peaks and their walks are those of the staged kernel.
+// Lines too long to stage (1-D signals beyond the staged capacity): a CTA takes one of gridDim.x parts
+// of a line's samples, reads samples from global memory (L1 / L2) and keeps the whole line's 32-sample
+// block extremes in shared memory (a warp per block); the peaks and their walks are those of the
+// staged kernel.
 template <class T>
 __global__ void __launch_bounds__(kThreads) flags_long(Geom g, const T* __restrict__ r, const T* __restrict__ tau,
                                                        uint8_t* __restrict__ flags, Elem* el, const int32_t* run) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int32_t count_s;
+  __shared__ uint32_t queue_s[kThreads / 32][kPeakQueue];
   const int64_t b = blockIdx.y;
   if (run && !run[b]) return;
-  const int64_t row = blockIdx.x;
   const int32_t n = elem_len(g, b);
+  int32_t s_first, s_end;
+  part_of_line(n, &s_first, &s_end, static_cast<int32_t>(gridDim.x), static_cast<int32_t>(blockIdx.x));
+  if (s_first >= s_end) return;
   const int32_t nb = (n + kBlk - 1) / kBlk;
   T* bmin = reinterpret_cast<T*>(smem_raw);
   T* bmax = bmin + nb;
-  const int64_t base = b * g.field + row * g.pitch;
+  const int64_t base = b * g.field;
   const T* line = r + base;
   if (threadIdx.x == 0) count_s = 0;
-  for (int32_t c = threadIdx.x; c < nb; c += blockDim.x) {
-    const int32_t len = min(kBlk, n - c * kBlk);
-    const T* xb = line + c * kBlk;
-    T mn = xb[0], mx = mn;
-    for (int32_t i = 1; i < len; ++i) {
-      const T v = xb[i];
-      mn = (v < mn || v != v) ? v : mn;
-      mx = (v > mx || v != v) ? v : mx;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int32_t c = warp; c < nb; c += kThreads / 32) {
+    const T v = line[min(c * kBlk + lane, n - 1)];
+    T mn = v, mx = v;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      const T a = __shfl_xor_sync(0xffffffffu, mn, d), z = __shfl_xor_sync(0xffffffffu, mx, d);
+      mn = (a < mn || a != a) ? a : mn;
+      mx = (z > mx || z != z) ? z : mx;
     }
-    bmin[c] = mn;
-    bmax[c] = mx;
+    if (lane == 0) {
+      bmin[c] = mn;
+      bmax[c] = mx;
+    }
   }
   __syncthreads();
   const auto at_k = [line](int32_t k) { return line[k]; };
-  int mine = 0;
-  for (int32_t s = 1 + threadIdx.x; s <= n - 2; s += blockDim.x) {
-    const T cur = line[s], prev = line[s - 1];
-    if (!(prev < cur || prev > cur)) continue;
-    // the run of samples equal to cur from s: samples of s's block, then whole blocks of cur
-    int32_t e;
-    {
-      const int32_t lim = min((s / kBlk) * kBlk + kBlk - 1, n - 1);
-      int32_t k = s + 1;
-      while (k <= lim && line[k] == cur) ++k;
-      if (k <= lim || k >= n) {
-        e = k - 1;
-      } else {
-        e = n - 1;
-        for (int32_t c = k / kBlk; c < nb; ++c) {
-          if (bmin[c] == cur && bmax[c] == cur) continue;
-          k = c * kBlk;
-          while (line[k] == cur) ++k;
-          e = k - 1;
-          break;
-        }
-      }
-    }
-    if (e > n - 2) continue;
-    const T nxt = line[e + 1];
-    const bool is_max = prev < cur && nxt < cur;
-    const bool is_min = prev > cur && nxt > cur;
-    if (!is_max && !is_min) continue;
-    const int32_t pk = (s + e) / 2;
-    const T tp = tau[base + pk];
-    const bool sig = is_max ? side_falls<true, -1>(at_k, n, pk, cur, tp, bmax, bmin) && side_falls<true, 1>(at_k, n, pk, cur, tp, bmax, bmin)
-                            : side_falls<false, -1>(at_k, n, pk, cur, tp, bmin, bmax) && side_falls<false, 1>(at_k, n, pk, cur, tp, bmin, bmax);
-    if (sig) {
+  int mine = 0, held = 0;
+  uint32_t* queue = queue_s[warp];
+  const auto judge = [&](uint32_t entry) {
+    const int32_t pk = static_cast<int32_t>(entry & 0xffffffu);
+    if (peak_counts<T>(at_k, n, pk, static_cast<int>(entry >> 30), tau[base + pk], bmin, bmax)) {
       flags[base + pk] |= static_cast<uint8_t>(1u);
       ++mine;
     }
+  };
+  for (int32_t s0 = s_first + 32 * warp; s0 < s_end; s0 += kThreads) {
+    int kind = 0;
+    int32_t pk = 0;
+    if (s0 + lane < s_end) kind = peak_at<T>(at_k, n, nb, s0 + lane, bmin, bmax, &pk);
+    push_peaks(queue, held, kind != 0, static_cast<uint32_t>(pk) | static_cast<uint32_t>(kind) << 30, judge);
   }
+  drain_peaks(queue, held, judge);
   for (int d = 16; d > 0; d >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, d);
-  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&count_s, mine);
+  if (lane == 0 && mine) atomicAdd(&count_s, mine);
   __syncthreads();
   if (threadIdx.x == 0 && count_s) {
     atomicAdd(reinterpret_cast<unsigned long long*>(&el[b].ext[0]), static_cast<unsigned long long>(count_s));
@@ -1148,20 +1215,33 @@ void sig_flags(cudaStream_t s, const Geom& g, const T* r, const T* tau, uint8_t*
   int optin = 0, dev = 0;
   EDAB_CUDA(cudaGetDevice(&dev));
   EDAB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const size_t cap = static_cast<size_t>(optin) - 2048;
+  const size_t cap = static_cast<size_t>(optin) - 4096;  // (the kernels' static shared memory)
   once_on_device(reinterpret_cast<const void*>(flags_pass<T>), [&] {  // the limit is per device
     EDAB_CUDA(cudaFuncSetAttribute(flags_pass<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cap)));
   });
+  int sms = 148;
+  EDAB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   for (int a = 0; a < g.dim; ++a) {
     const int32_t n = g.n[a];
     if (n < 3) continue;
+    const bool rows = a == g.dim - 1;
     const int32_t nb = (n + kBlk - 1) / kBlk;
+    int64_t outer = 1;
+    for (int ax = 0; ax < a; ++ax) outer *= g.n[ax];
+    const auto groups_of = [&](int p) { return rows ? (g.rows + p - 1) / p : outer * ((g.stride[a] + p - 1) / p); };
     int P;
-    if (a == g.dim - 1) P = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({static_cast<int64_t>(8192 / n), g.rows, 64})));
+    if (rows) P = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({static_cast<int64_t>(8192 / n), g.rows, 64})));
     else P = static_cast<int>(std::min<int64_t>(16, g.stride[a]));  // a power of two (stride: a multiple of 32)
+    // fewer lines per CTA while the launch would leave SMs without one (a column panel keeps whole
+    // sectors)
+    while (P > (rows ? 1 : 8) && groups_of(P) * g.batch < 2 * sms) P /= 2;
     const int32_t LX = (n + ((n - 1) >> 5) + 1) | 1;  // padded line words, odd
     const auto bytes = [&](int p) { return static_cast<size_t>(p) * (LX + 2 * nb) * sizeof(T); };
-    while (P > 1 && bytes(P) > cap) P = a == g.dim - 1 ? P - 1 : P / 2;
+    while (P > 1 && bytes(P) > cap) P = rows ? P - 1 : P / 2;
+    // a 1-D line's parts: at least 512 samples each, about one CTA per SM in all
+    const int32_t parts = g.dim == 1 ? static_cast<int32_t>(std::clamp<int64_t>(
+                                           std::min<int64_t>(n / 512, sms / std::max<int64_t>(1, g.batch)), 1, 64))
+                                     : 1;
     if (bytes(P) > cap) {
       // a 1-D line beyond the staged capacity: samples from global memory, block extremes staged
       const size_t ext_bytes = static_cast<size_t>(2) * nb * sizeof(T);
@@ -1169,21 +1249,14 @@ void sig_flags(cudaStream_t s, const Geom& g, const T* r, const T* tau, uint8_t*
       once_on_device(reinterpret_cast<const void*>(flags_long<T>), [&] {
         EDAB_CUDA(cudaFuncSetAttribute(flags_long<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cap)));
       });
-      flags_long<T><<<dim3(static_cast<unsigned>(g.rows), static_cast<unsigned>(g.batch)), kThreads, ext_bytes, s>>>(
+      const int64_t fill = std::clamp<int64_t>((8 * static_cast<int64_t>(sms) + g.batch - 1) / g.batch, 1, 16);
+      flags_long<T><<<dim3(static_cast<unsigned>(fill), static_cast<unsigned>(g.batch)), kThreads, ext_bytes, s>>>(
           g, r, tau, flags, el, run);
       EDAB_LAUNCH("flags_long");
       continue;
     }
-    int64_t groups;
-    if (a == g.dim - 1) {
-      groups = (g.rows + P - 1) / P;
-    } else {
-      int64_t outer = 1;
-      for (int ax = 0; ax < a; ++ax) outer *= g.n[ax];
-      groups = outer * ((g.stride[a] + P - 1) / P);
-    }
-    flags_pass<T><<<dim3(static_cast<unsigned>(groups), static_cast<unsigned>(g.batch)), kThreads, bytes(P), s>>>(
-        g, a, r, tau, flags, el, run, P, LX);
+    flags_pass<T><<<dim3(static_cast<unsigned>(groups_of(P) * parts), static_cast<unsigned>(g.batch)), kThreads, bytes(P), s>>>(
+        g, a, r, tau, flags, el, run, P, LX, parts);
     EDAB_LAUNCH("flags_pass");
   }
 }
