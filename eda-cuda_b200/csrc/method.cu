@@ -394,13 +394,30 @@ __device__ __forceinline__ T gather_op(T acc, T v, bool second) {
   else return max_c(acc, v);
 }
 
+// What a gather stores besides (or instead of) its values: the pointwise step that follows it in the
+// sift, so that the values are not written and read again for it (64 images of 512 x 512: the middles,
+// halves, ranges, weights and differences took 2.9 ms per decomposition in kernels of their own; the
+// gathers themselves, bound by their interpolated reads, take as long as before). Null pointers: not
+// stored.
+template <class T>
+struct GatherOut {
+  T *out0, *out1;     // the gathered values
+  T* mid;             // max and min: (u + l) / 2
+  T* half;            // max and min: (u - l) / 2
+  T* range;           // max and min: max(u - l, 0)
+  const T* from;      // box: out0 = from - value
+  int32_t clip01;     // box: out0 = the value clipped to [0, 1]
+  const T* weight_of; // max: out0 = clip((clip(R / U, 0, 1) - t0) / den, 0, 1), R = weight_of, U the value
+  T t0, den;
+};
+
 template <class T, int D, int OP>
 __global__ void __launch_bounds__(kThreads, EDAB_GATHER_CTAS) gather_kernel(Geom g, const Elem* __restrict__ el,
                                                          const int32_t* __restrict__ run, const uint8_t* __restrict__ lo,
                                                          const T* __restrict__ t, const T* __restrict__ o0,
                                                          const T* __restrict__ o1, const T* __restrict__ o2,
                                                          const T* __restrict__ rung0, const T* __restrict__ rung1,
-                                                         T* __restrict__ out0, T* __restrict__ out1) {
+                                                         GatherOut<T> go) {
   const int64_t fe = g.batch * g.field;
   for (int64_t b = blockIdx.y; b < g.batch; b += gridDim.y) {
     if (!run[b]) continue;
@@ -468,15 +485,38 @@ __global__ void __launch_bounds__(kThreads, EDAB_GATHER_CTAS) gather_kernel(Geom
           r1 = use0 ? add_rn(r1, v1) : v1;
         }
       }
-      out0[at] = r0;
-      if constexpr (OP == 2) out1[at] = r1;
+      if constexpr (OP == 2) {
+        if (go.out0) go.out0[at] = r0;
+        if (go.out1) go.out1[at] = r1;
+        go.mid[at] = mul_rn(T(0.5), add_rn(r0, r1));
+        if (go.half) go.half[at] = mul_rn(T(0.5), sub_rn(r0, r1));
+        if (go.range) go.range[at] = np_max(sub_rn(r0, r1), T(0));
+      } else if constexpr (OP == 3) {
+        if (go.from) r0 = sub_rn(go.from[at], r0);
+        else if (go.clip01) r0 = clip(r0, T(0), T(1));
+        go.out0[at] = r0;
+      } else {
+        if (go.weight_of) {
+          T rho = T(0);
+          if (static_cast<double>(r0) > el[b].tol) rho = clip(div_rn(go.weight_of[at], r0), T(0), T(1));
+          r0 = clip(div_rn(sub_rn(rho, go.t0), go.den), T(0), T(1));
+        }
+        go.out0[at] = r0;
+      }
     }
   }
 }
 
-template <class T, int D>
-__global__ void __launch_bounds__(kThreads) sift_step_kernel(Geom g, int32_t j, Elem* el, const T* __restrict__ r,
-                                                            const T* __restrict__ h, const T* __restrict__ mh,
+// One sift j >= 2 of the sifting elements: the mean blended from the normalised one (e M, clipped to
+// the plain envelopes) and the plain one by the weight g, the damped step hn = h - a mean, and the
+// maxima of |r - hn| and |hn| for the guard.
+template <class T>
+struct SiftBlend {
+  const T *g, *e, *up, *lo, *plain, *M;
+};
+template <class T>
+__global__ void __launch_bounds__(kThreads) sift_step_kernel(Geom g, Elem* el, const T* __restrict__ r,
+                                                            const T* __restrict__ h, SiftBlend<T> m,
                                                             const T* __restrict__ a, T* __restrict__ hn) {
   for (int64_t b = blockIdx.y; b < g.batch; b += gridDim.y) {
     const Elem& e = el[b];
@@ -487,28 +527,25 @@ __global__ void __launch_bounds__(kThreads) sift_step_kernel(Geom g, int32_t j, 
          v += static_cast<int64_t>(gridDim.x) * blockDim.x) {
       if (pitch_col(g, v) >= nl) continue;
       const int64_t i = b * g.field + v;
-      T m = mh[i];
-      if (j >= 1) m = mul_rn(a[i], m);
-      const T x = sub_rn(h[i], m);
+      const T w = m.g[i];
+      const T normal = clip(mul_rn(m.e[i], m.M[i]), m.lo[i], m.up[i]);
+      const T mean = add_rn(mul_rn(w, normal), mul_rn(sub_rn(T(1), w), m.plain[i]));
+      const T x = sub_rn(h[i], mul_rn(a[i], mean));
       hn[i] = x;
-      if (j >= 1) {
-        const uint64_t br = abs_bits(sub_rn(r[i], x));
-        const uint64_t bh = abs_bits(x);
-        m_res = br > m_res ? br : m_res;
-        m_h = bh > m_h ? bh : m_h;
-      }
+      const uint64_t br = abs_bits(sub_rn(r[i], x));
+      const uint64_t bh = abs_bits(x);
+      m_res = br > m_res ? br : m_res;
+      m_h = bh > m_h ? bh : m_h;
     }
-    if (j >= 1) {
-      for (int o = 16; o > 0; o >>= 1) {
-        const uint64_t u1 = __shfl_xor_sync(0xffffffffu, m_res, o);
-        const uint64_t u2 = __shfl_xor_sync(0xffffffffu, m_h, o);
-        m_res = u1 > m_res ? u1 : m_res;
-        m_h = u2 > m_h ? u2 : m_h;
-      }
-      if ((threadIdx.x & 31) == 0) {
-        if (m_res) atomicMax(reinterpret_cast<unsigned long long*>(&el[b].gmax_res_bits), static_cast<unsigned long long>(m_res));
-        if (m_h) atomicMax(reinterpret_cast<unsigned long long*>(&el[b].gmax_h_bits), static_cast<unsigned long long>(m_h));
-      }
+    for (int o = 16; o > 0; o >>= 1) {
+      const uint64_t u1 = __shfl_xor_sync(0xffffffffu, m_res, o);
+      const uint64_t u2 = __shfl_xor_sync(0xffffffffu, m_h, o);
+      m_res = u1 > m_res ? u1 : m_res;
+      m_h = u2 > m_h ? u2 : m_h;
+    }
+    if ((threadIdx.x & 31) == 0) {
+      if (m_res) atomicMax(reinterpret_cast<unsigned long long*>(&el[b].gmax_res_bits), static_cast<unsigned long long>(m_res));
+      if (m_h) atomicMax(reinterpret_cast<unsigned long long*>(&el[b].gmax_h_bits), static_cast<unsigned long long>(m_h));
     }
   }
 }
@@ -540,8 +577,7 @@ class Engine {
   // fields
   T *r_, *L_, *Lp_, *h_, *t_, *tau_, *tmp_, *om_, *om2_, *tmp0_, *tmp1_;
   T *n_[kMaxDim], *coh_, *o_[kMaxDim];
-  T *m_, *u_, *l_, *mid_, *R_, *U1_, *U2_, *gw_, *a_, *plain_, *up_, *lo_f_, *hd_, *e0_, *emax_, *emin_, *gk_, *e_,
-      *q_, *Mn_, *u2_, *l2_, *hn_;
+  T *mid_, *R_, *U1_, *U2_, *gw_, *a_, *plain_, *up_, *lo_f_, *hd_, *e0_, *emax_, *emin_, *gk_, *e_, *q_, *Mn_, *hn_;
   T *rung0_, *rung1_;
   T* owork_;
   uint8_t *flags_, *ff_, *P_[2], *Pacc_, *A_, *lo_, *marks_, *selm_;
@@ -583,8 +619,8 @@ class Engine {
   void orientation_and_build();
   void store_orientation();
   bool ladder_and_weights(int32_t* n_rungs_max);
-  void op(int which, const T* in, T* out0, T* out1, int32_t n_rungs_max);
-  void envelope_mean(const T* h, T* m, T* u, T* l, int32_t nrm);
+  void op(int which, const T* in, const GatherOut<T>& out, int32_t n_rungs_max);
+  void envelope_mean(const T* h, const GatherOut<T>& ext, const GatherOut<T>& mean, int32_t nrm);
   void sifts(int32_t nrm);
   bool commit();
 };
@@ -601,9 +637,9 @@ void Engine<T>::bind(Workspace& ws) {
     o_[a] = a < g_.dim && g_.dim >= 2 ? fld() : nullptr;
   }
   coh_ = fld();
-  m_ = fld(); u_ = fld(); l_ = fld(); mid_ = fld(); R_ = fld(); U1_ = fld(); U2_ = fld(); gw_ = fld(); a_ = fld();
+  mid_ = fld(); R_ = fld(); U1_ = fld(); U2_ = fld(); gw_ = fld(); a_ = fld();
   plain_ = fld(); up_ = fld(); lo_f_ = fld(); hd_ = fld(); e0_ = fld(); emax_ = fld(); emin_ = fld(); gk_ = fld();
-  e_ = fld(); q_ = fld(); Mn_ = fld(); u2_ = fld(); l2_ = fld(); hn_ = fld();
+  e_ = fld(); q_ = fld(); Mn_ = fld(); hn_ = fld();
   rung0_ = ws.take<T>(F * kMaxRungs);
   rung1_ = ws.take<T>(F * kMaxRungs);
   owork_ = g_.dim >= 2 ? ws.take<T>(static_cast<size_t>(orient_work_samples(g_))) : nullptr;
@@ -671,59 +707,40 @@ void Engine<T>::tau_field(const int32_t* run, bool floor2, T* tau) {
   a.rungs = 1;
   a.epi.kind = BoxEpi::kDetSq;
   a.epi.aux = r_;
+  a.epi.run = run;
   cube<T>(s_, g_, CubeOp::kBox, a);
-  cube_simple<T>(s_, g_, CubeOp::kBox, tmp_, tau, nullptr, win(kWl));
-  const Ctl c = c_;
-  Elem* el = el_;
-  const int32_t* wd = win(kWd);
-  for_voxels(s_, g_, [=] __device__(int64_t b) { return run[b] && wd[b] >= 1; },
-             [=] __device__(int64_t b, int64_t, int64_t i) {
-               const T be = tau[i];
-               const double sn = el[b].sigma_n;
-               if (!(isfinite(be) && isfinite(sn))) el[b].nonfinite = 1;
-               const T lev = sqrt_rn<T>(be > T(0) ? be : T(0));
-               const double f = __dmul_rn(c.sig_noise, sn);
-               const double fl = f > 0.0 ? f : 0.0;
-               const double ld = static_cast<double>(lev);
-               double t = __dmul_rn(c.sig_theta, ld > fl ? ld : fl);
-               const double tl = el[b].tol;
-               t = t > tl ? t : tl;
-               if (floor2) {
-                 const double f2 = __dmul_rn(c.fine_theta, el[b].sigma_x);
-                 t = t > f2 ? t : f2;
-               }
-               tau[i] = static_cast<T>(t);
-             });
+  a.in = tmp_;
+  a.out0 = tau;
+  a.win = win(kWl);
+  a.epi.kind = BoxEpi::kTau;
+  a.epi.aux = nullptr;
+  a.epi.el = el_;
+  a.epi.sig_noise = c_.sig_noise;
+  a.epi.sig_theta = c_.sig_theta;
+  a.epi.fine_theta = c_.fine_theta;
+  a.epi.floor2 = floor2;
+  cube<T>(s_, g_, CubeOp::kBox, a);
 }
 
 // The raw window (cpp/src/method/stats_fields.cu:340-369): rho_a = Box_w (bit a of flags), om =
 // 2 kappa / max(sqrt(sum rho_a^2), tiny) where the density is positive, +inf elsewhere.
 template <class T>
 void Engine<T>::raw_window(const uint8_t* flags, const int32_t* w, const int32_t* run, T* om, T* tmp) {
-  const T two_kappa = static_cast<T>(2.0 * c_.kappa);
-  const T tiny = static_cast<T>(c_.tiny);
-  const int D = g_.dim;
-  for (int a = 0; a < D; ++a) {
+  for (int a = 0; a < g_.dim; ++a) {
     CubeArgs<T> ca{};
     ca.src_bits = flags;
     ca.bit = a;
     ca.out0 = tmp;
     ca.win = w;
     ca.rungs = 1;
+    ca.epi.kind = BoxEpi::kRho;
+    ca.epi.aux = a > 0 ? om : nullptr;
+    ca.epi.out = om;
+    ca.epi.run = run;
+    ca.epi.finish = a == g_.dim - 1;
+    ca.epi.two_kappa = static_cast<T>(2.0 * c_.kappa);
+    ca.epi.tiny = static_cast<T>(c_.tiny);
     cube<T>(s_, g_, CubeOp::kBox, ca);
-    const bool last = a == D - 1;
-    for_voxels(s_, g_, [=] __device__(int64_t b) { return run[b] && w[b] >= 1; },
-               [=] __device__(int64_t, int64_t, int64_t i) {
-                 const T rho = tmp[i];
-                 const T sq = mul_rn(rho, rho);
-                 const T acc = a == 0 ? sq : add_rn(om[i], sq);
-                 if (!last) {
-                   om[i] = acc;
-                   return;
-                 }
-                 const T dens = sqrt_rn<T>(acc);
-                 om[i] = dens > T(0) ? div_rn<T>(two_kappa, dens > tiny ? dens : tiny) : inf_t<T>();
-               });
   }
 }
 
@@ -784,8 +801,14 @@ void Engine<T>::scale_field() {
     }
     L[i] = log_t<T>(static_cast<T>(v));
   });
-  cube_simple<T>(s_, g_, CubeOp::kBox, L, L, nullptr, wW);
-  for_voxels(s_, g_, runW, [=] __device__(int64_t, int64_t, int64_t i) { L[i] = exp_t<T>(L[i]); });
+  CubeArgs<T> la{};
+  la.in = L;
+  la.out0 = L;
+  la.win = wW;
+  la.rungs = 1;
+  la.epi.kind = BoxEpi::kExp;
+  la.epi.run = on;
+  cube<T>(s_, g_, CubeOp::kBox, la);
 }
 
 // The per-voxel floor of modes k >= 1 (cpp/src/method/stats_scale.cu:169-201, 249-268).
@@ -1120,7 +1143,7 @@ bool Engine<T>::ladder_and_weights(int32_t* n_rungs_max) {
 // An operator over every used rung: the rung cubes (one launch per pass for all rungs; the first
 // pass stages the input once), then one gather per voxel.
 template <class T>
-void Engine<T>::op(int which, const T* in, T* out0, T* out1, int32_t nrm) {
+void Engine<T>::op(int which, const T* in, const GatherOut<T>& out, int32_t nrm) {
   CubeArgs<T> a{};
   a.in = in;
   a.out0 = rung0_;
@@ -1138,7 +1161,7 @@ void Engine<T>::op(int which, const T* in, T* out0, T* out1, int32_t nrm) {
   const T* o1 = o_[1];
   const T* o2 = o_[2];
 #define EDAB_GATHER(D, OP) \
-  gather_kernel<T, D, OP><<<grid, kThreads, 0, s_>>>(g_, el_, on, lo_, t_, o0, o1, o2, rung0_, rung1_, out0, out1)
+  gather_kernel<T, D, OP><<<grid, kThreads, 0, s_>>>(g_, el_, on, lo_, t_, o0, o1, o2, rung0_, rung1_, out)
   if (g_.dim == 1) {
     if (which == 0) EDAB_GATHER(1, 0); else if (which == 2) EDAB_GATHER(1, 2); else EDAB_GATHER(1, 3);
   } else if (g_.dim == 2) {
@@ -1150,14 +1173,14 @@ void Engine<T>::op(int which, const T* in, T* out0, T* out1, int32_t nrm) {
   EDAB_LAUNCH("gather_kernel");
 }
 
+// The mean envelope of h: the extremes with what `ext` stores of them (the middle always), then the box
+// operator of the middle with what `mean` stores.
 template <class T>
-void Engine<T>::envelope_mean(const T* h, T* m, T* u, T* l, int32_t nrm) {
-  op(2, h, u, l, nrm);
-  T* mid = mid_;
-  const int32_t* on = mask(kOn);
-  for_voxels(s_, g_, [=] __device__(int64_t b) { return on[b] != 0; },
-             [=] __device__(int64_t, int64_t, int64_t i) { mid[i] = mul_rn(T(0.5), add_rn(u[i], l[i])); });
-  op(3, mid, m, nullptr, nrm);
+void Engine<T>::envelope_mean(const T* h, const GatherOut<T>& ext, const GatherOut<T>& mean, int32_t nrm) {
+  GatherOut<T> e = ext;
+  e.mid = mid_;
+  op(2, h, e, nrm);
+  op(3, mid_, mean, nrm);
 }
 
 // Sift 1, the continuation weight, sifts 2..S with G1 and the guard
@@ -1170,11 +1193,13 @@ void Engine<T>::sifts(int32_t nrm) {
   const auto runOn = [=] __device__(int64_t b) { return on[b] != 0; };
   T* r = r_;
   T* h = h_;
-  envelope_mean(r_, m_, u_, l_, nrm);
+  // sift 1: h = r - mean envelope; the range R = max(Dil r - Ero r, 0) for the continuation weight
   {
-    const T* m = m_;
-    for_voxels(s_, g_, [=] __device__(int64_t b) { return el[b].status == kActive && el[b].sifting; },
-               [=] __device__(int64_t, int64_t, int64_t i) { h[i] = sub_rn(r[i], m[i]); });
+    GatherOut<T> ext{}, mean{};
+    if (c_.sifts > 1) ext.range = R_;
+    mean.out0 = h;
+    mean.from = r;
+    envelope_mean(r_, ext, mean, nrm);
     for_elements(s_, B_, [=] __device__(int64_t b) {
       if (el[b].status == kActive && el[b].sifting) el[b].n_sifts += 1;
       el[b].gmax_res_bits = 0;
@@ -1182,54 +1207,43 @@ void Engine<T>::sifts(int32_t nrm) {
     });
   }
   if (c_.sifts <= 1) return;
-  // the continuation weight: R = max(Dil r - Ero r, 0), U = Dil^u R, g = ramp(R / U), a = clip(Avg^s g)
-  {
-    T* R = R_;
-    const T* u = u_;
-    const T* l = l_;
-    for_voxels(s_, g_, runOn, [=] __device__(int64_t, int64_t, int64_t i) { R[i] = np_max(sub_rn(u[i], l[i]), T(0)); });
-  }
+  // the continuation weight: U = Dil^u R, g = ramp(R / U), a = clip(Avg^s g)
   const T* U = R_;
   T* pp[2] = {U1_, U2_};
   for (int32_t i = 0; i < c_.u; ++i) {
-    op(0, U, pp[i & 1], nullptr, nrm);
+    GatherOut<T> out{};
+    out.out0 = pp[i & 1];
+    if (i + 1 == c_.u) {
+      const double dd = c.t1 - c.t0;
+      out.out0 = gw_;
+      out.weight_of = R_;
+      out.t0 = static_cast<T>(c.t0);
+      out.den = static_cast<T>(dd >= 1e-12 ? dd : 1e-12);
+    }
+    op(0, U, out, nrm);
     U = pp[i & 1];
-  }
-  {
-    const T* R = R_;
-    T* gw = gw_;
-    const T t0 = static_cast<T>(c.t0);
-    const double dd = c.t1 - c.t0;
-    const T den = static_cast<T>(dd >= 1e-12 ? dd : 1e-12);
-    for_voxels(s_, g_, runOn, [=] __device__(int64_t b, int64_t, int64_t i) {
-      const double tol = el[b].tol;
-      const T Uv = U[i];
-      T rho = T(0);
-      if (static_cast<double>(Uv) > tol) rho = clip(div_rn(R[i], Uv), T(0), T(1));
-      gw[i] = clip(div_rn(sub_rn(rho, t0), den), T(0), T(1));
-    });
   }
   const T* cur = gw_;
   for (int32_t i = 0; i < c_.s; ++i) {
-    T* dst = (i + 1 < c_.s) ? (cur == U1_ ? U2_ : U1_) : a_;
-    op(3, cur, dst, nullptr, nrm);
-    cur = dst;
-  }
-  {
-    T* a = a_;
-    for_voxels(s_, g_, runOn, [=] __device__(int64_t, int64_t, int64_t i) { a[i] = clip(a[i], T(0), T(1)); });
+    GatherOut<T> out{};
+    out.clip01 = i + 1 == c_.s;
+    out.out0 = out.clip01 ? a_ : (cur == U1_ ? U2_ : U1_);
+    op(3, cur, out, nrm);
+    cur = out.out0;
   }
   // sifts 2..S
   const int32_t* wW = win(kW);
   for (int32_t j = 1; j < c_.sifts; ++j) {
-    envelope_mean(h_, plain_, up_, lo_f_, nrm);
     {
-      T* hd = hd_;
-      const T* up = up_;
-      const T* lo = lo_f_;
-      for_voxels(s_, g_, runOn, [=] __device__(int64_t, int64_t, int64_t i) { hd[i] = mul_rn(T(0.5), sub_rn(up[i], lo[i])); });
+      GatherOut<T> ext{}, mean{}, half{};
+      ext.out0 = up_;
+      ext.out1 = lo_f_;
+      ext.half = hd_;
+      mean.out0 = plain_;
+      envelope_mean(h_, ext, mean, nrm);
+      half.out0 = e0_;
+      op(3, hd_, half, nrm);
     }
-    op(3, hd_, e0_, nullptr, nrm);
     cube_simple<T>(s_, g_, CubeOp::kMaxMin, e0_, emax_, emin_, wW);
     {
       T* kr = emax_;
@@ -1246,10 +1260,15 @@ void Engine<T>::sifts(int32_t nrm) {
         kr[i] = clip(div_rn(sub_rn(kap, k0), kden), T(0), T(1));
       });
     }
-    cube_simple<T>(s_, g_, CubeOp::kBox, emax_, gk_, nullptr, wW);
     {
-      T* gk = gk_;
-      for_voxels(s_, g_, runOn, [=] __device__(int64_t, int64_t, int64_t i) { gk[i] = clip(gk[i], T(0), T(1)); });
+      CubeArgs<T> ka{};
+      ka.in = emax_;
+      ka.out0 = gk_;
+      ka.win = wW;
+      ka.rungs = 1;
+      ka.epi.kind = BoxEpi::kClip;
+      ka.epi.run = on;
+      cube<T>(s_, g_, CubeOp::kBox, ka);
     }
     const T* esrc = e0_;
     for (int32_t i = 0; i < c_.anorm_smooth; ++i) {
@@ -1276,22 +1295,14 @@ void Engine<T>::sifts(int32_t nrm) {
         q[i] = div_rn(hh[i], ef);
       });
     }
-    envelope_mean(q_, Mn_, u2_, l2_, nrm);
     {
-      T* Mn = Mn_;
-      const T* gk = gk_;
-      const T* e = e_;
-      const T* up = up_;
-      const T* lo = lo_f_;
-      const T* plain = plain_;
-      for_voxels(s_, g_, runOn, [=] __device__(int64_t, int64_t, int64_t i) {
-        const T w = gk[i];
-        const T mA = clip(mul_rn(e[i], Mn[i]), lo[i], up[i]);
-        Mn[i] = add_rn(mul_rn(w, mA), mul_rn(sub_rn(T(1), w), plain[i]));
-      });
+      GatherOut<T> ext{}, mean{};
+      mean.out0 = Mn_;
+      envelope_mean(q_, ext, mean, nrm);
     }
     const dim3 grid = voxel_grid(g_);
-    sift_step_kernel<T, 1><<<grid, kThreads, 0, s_>>>(g_, j, el_, r_, h_, Mn_, a_, hn_);
+    const SiftBlend<T> blend{gk_, e_, up_, lo_f_, plain_, Mn_};
+    sift_step_kernel<T><<<grid, kThreads, 0, s_>>>(g_, el_, r_, h_, blend, a_, hn_);
     EDAB_LAUNCH("sift_step_kernel");
     {
       T* hh = h_;
@@ -1629,6 +1640,10 @@ void Engine<T>::run(const T* x, T* rows_out, int32_t* hist_scale, int32_t* hist_
 }
 
 // ---------------------------------------------------------------------------------------------
+// What a call of this geometry is accounted for, in the device memory that the batch is chunked by and
+// in the fixed scratch of the calls that allocate nothing: 24 fields of a sift and, for the longest
+// 1-D lines, a fold scratch. A run takes less (18 fields; the long lines' scratch lies in the fields
+// left over, the chunk totals of their box passes in the rungs' minima, which no box pass holds).
 template <class T>
 size_t engine_bytes(const Geom& g) {
   const size_t F = static_cast<size_t>(g.batch * g.field);
@@ -1638,7 +1653,7 @@ size_t engine_bytes(const Geom& g) {
   if (D >= 2) b += static_cast<size_t>(orient_work_samples(g)) * sizeof(T);
   b += static_cast<size_t>(g.batch) * (sizeof(Elem) + 4 * (kSlots + kMasks + kMaxRungs) + 8 * 10 + 64);
   b += select_scratch_bytes(g) + totals_scratch_bytes(g);
-  b += fold_scratch_bytes(g, sizeof(T)) + long_line_scratch_bytes(g, sizeof(T));
+  b += fold_scratch_bytes(g, sizeof(T));
   b += 160 * 256;  // every take is rounded up to 256 bytes
   return b;
 }
