@@ -584,6 +584,67 @@ int64_t orient_work_samples(const Geom& g) {
   return g.batch * (3 * orient_layout_samples(g) + static_cast<int64_t>(D + D * (D + 1) / 2) * g.field);
 }
 
+namespace {
+
+// The Riesz multiplier of component (kind, a, b) at the spectrum index k (riesz_mult, orientation.cu:
+// 116-127): 0 R1_a, 1 R2_aa, 2 R2_ab, 3 D_a f, 4 D_b R_a; 0 at the DC.
+template <int D>
+__device__ __forceinline__ double riesz_mult(const Geom& g, int kind, int a, int b, const int32_t* k) {
+  double u[kMaxDim];
+  const double rad = dct_freq<D>(g, k, u);
+  if (!(rad > 0.0)) return 0.0;
+  // (u at a run-time index would lie in local memory)
+  const double va = a == 0 ? u[0] : (D < 3 || a == 1 ? u[D > 1 ? 1 : 0] : u[D > 2 ? 2 : 0]);
+  const double vb = b == 0 ? u[0] : (D < 3 || b == 1 ? u[D > 1 ? 1 : 0] : u[D > 2 ? 2 : 0]);
+  const double inv = __ddiv_rn(1.0, rad);
+  const double ua = __dmul_rn(va, inv);
+  if (kind == 0) return ua;
+  if (kind == 1) return __dmul_rn(-ua, ua);
+  if (kind == 3) return -va;
+  if (kind == 4) return a == b ? __dmul_rn(va, ua) : -__dmul_rn(va, __dmul_rn(vb, inv));
+  return __dmul_rn(ua, __dmul_rn(vb, inv));
+}
+
+// Y = component (kind, a, b) of the spectra X of the elements that run. The multiplier (a double square
+// root and division) depends on the frequency alone: a thread forms it once for its frequency of
+// kRieszPer elements, so the pass is bound by reading X and writing Y.
+constexpr int kRieszPer = 8;
+template <class T, int D>
+__global__ void __launch_bounds__(256) riesz_spectrum(Geom g, int kind, int a, int b, const int32_t* __restrict__ run,
+                                                      const T* __restrict__ X, T* __restrict__ Y) {
+  for (int64_t v = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; v < g.field;
+       v += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    int32_t k[kMaxDim];
+    if (!voxel_coords_d<D>(g, v, g.n[D - 1], k)) continue;
+    const double m = riesz_mult<D>(g, kind, a, b, k);
+    for (int64_t e0 = static_cast<int64_t>(blockIdx.y) * kRieszPer; e0 < g.batch;
+         e0 += static_cast<int64_t>(gridDim.y) * kRieszPer) {
+      T x[kRieszPer];
+#pragma unroll
+      for (int j = 0; j < kRieszPer; ++j) x[j] = e0 + j < g.batch ? X[(e0 + j) * g.field + v] : T(0);
+#pragma unroll
+      for (int j = 0; j < kRieszPer; ++j) {
+        if (e0 + j < g.batch && run[e0 + j]) {
+          Y[(e0 + j) * g.field + v] = static_cast<T>(__dmul_rn(m, static_cast<double>(x[j])));
+        }
+      }
+    }
+  }
+}
+template <class T>
+void launch_riesz(cudaStream_t s, const Geom& g, int kind, int a, int b, const int32_t* run, const T* X, T* Y) {
+  dim3 grid = voxel_grid(g, 1);
+  grid.y = static_cast<unsigned>(std::clamp<int64_t>((g.batch + kRieszPer - 1) / kRieszPer, 1, 65535));
+  switch (g.dim) {
+    case 1: riesz_spectrum<T, 1><<<grid, 256, 0, s>>>(g, kind, a, b, run, X, Y); break;
+    case 2: riesz_spectrum<T, 2><<<grid, 256, 0, s>>>(g, kind, a, b, run, X, Y); break;
+    default: riesz_spectrum<T, 3><<<grid, 256, 0, s>>>(g, kind, a, b, run, X, Y); break;
+  }
+  EDAB_LAUNCH("riesz_spectrum");
+}
+
+}  // namespace
+
 template <class T>
 void orientation(cudaStream_t s, const Geom& g, const OrientPlan& plan, const T* r, Elem* el, const int32_t* run,
                  T* const* n, T* coh, T* work, double two_sigma2, int32_t* err) {
@@ -640,23 +701,7 @@ void orientation(cudaStream_t s, const Geom& g, const OrientPlan& plan, const T*
     for (int a = 0; a < D; ++a) {
       for (int b2 = (kind == 0 ? a : a); b2 < (kind == 0 ? a + 1 : D); ++b2) {
         T* out = kind == 0 ? R1 + a * F : R2 + (p++) * F;
-        const int ca = a, cb = b2, ck = kind;
-        for_voxels(s, g, [=] __device__(int64_t bb) { return run[bb] != 0; },
-                   [=] __device__(int64_t, int64_t v, int64_t i) {
-                     int32_t k[kMaxDim];
-                     voxel_coords(gg, v, k);
-                     double u[kMaxDim];
-                     const double rad = gg.dim == 2 ? dct_freq<2>(gg, k, u) : dct_freq<3>(gg, k, u);
-                     double m = 0.0;
-                     if (rad > 0.0) {
-                       const double inv = __ddiv_rn(1.0, rad);
-                       const double ua = __dmul_rn(u[ca], inv);
-                       if (ck == 0) m = ua;
-                       else if (ca == cb) m = __dmul_rn(-ua, ua);
-                       else m = __dmul_rn(ua, __dmul_rn(u[cb], inv));
-                     }
-                     Y[i] = static_cast<T>(__dmul_rn(m, static_cast<double>(X[i])));
-                   });
+        launch_riesz<T>(s, g, kind == 0 ? 0 : (a == b2 ? 1 : 2), a, b2, run, X, Y);
         const int odd = kind == 0 ? (1 << a) : (a == b2 ? 0 : ((1 << a) | (1 << b2)));
         transform(Y, out, [odd](int ax) { return ((odd >> ax) & 1) ? 2 : 1; });
       }
@@ -676,36 +721,6 @@ void orientation(cudaStream_t s, const Geom& g, const OrientPlan& plan, const T*
 // m_ab = 2 n_a n_b); where A^2 > tiny: phase = atan2(q, f) (an angle that rounds to -pi is pi),
 // frequency = (f D_n q - q D_n f) / A^2; amplitude = sqrt(A^2) 2^exp, rounded once.
 namespace {
-
-// The Riesz multiplier of component (kind, a, b) at the spectrum index k (riesz_mult, orientation.cu:
-// 116-127): 0 R1_a, 1 R2_aa, 2 R2_ab, 3 D_a f, 4 D_b R_a; 0 at the DC.
-template <int D>
-__device__ __forceinline__ double riesz_mult(const Geom& g, int kind, int a, int b, const int32_t* k) {
-  double u[kMaxDim];
-  const double rad = dct_freq<D>(g, k, u);
-  if (!(rad > 0.0)) return 0.0;
-  const double inv = __ddiv_rn(1.0, rad);
-  const double ua = __dmul_rn(u[a], inv);
-  if (kind == 0) return ua;
-  if (kind == 1) return __dmul_rn(-ua, ua);
-  if (kind == 3) return -u[a];
-  if (kind == 4) return a == b ? __dmul_rn(u[a], ua) : -__dmul_rn(u[a], __dmul_rn(u[b], inv));
-  return __dmul_rn(ua, __dmul_rn(u[b], inv));
-}
-
-template <class T, int D>
-__global__ void __launch_bounds__(256) riesz_spectrum(Geom g, int kind, int a, int b, const T* __restrict__ X,
-                                                      T* __restrict__ Y) {
-  for (int64_t e = blockIdx.y; e < g.batch; e += gridDim.y) {
-    for (int64_t v = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; v < g.field;
-         v += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-      int32_t k[kMaxDim];
-      if (!voxel_coords_d<D>(g, v, g.n[D - 1], k)) continue;
-      const int64_t i = e * g.field + v;
-      Y[i] = static_cast<T>(__dmul_rn(riesz_mult<D>(g, kind, a, b, k), static_cast<double>(X[i])));
-    }
-  }
-}
 
 template <class T, int D>
 __global__ void __launch_bounds__(256) monogenic_kernel(Geom g, const T* __restrict__ f, const T* r1,
@@ -814,12 +829,7 @@ void monogenic_fields(cudaStream_t s, const Geom& g, const OrientPlan& plan, con
   transform_axes<T>(s, g, plan, Y, X, Z, Y, kinds, run, err);
   const dim3 grid = voxel_grid(g);
   auto component = [&](int kind, int a, int b, T* dst) {
-    switch (D) {
-      case 1: riesz_spectrum<T, 1><<<grid, 256, 0, s>>>(g, kind, a, b, X, Y); break;
-      case 2: riesz_spectrum<T, 2><<<grid, 256, 0, s>>>(g, kind, a, b, X, Y); break;
-      default: riesz_spectrum<T, 3><<<grid, 256, 0, s>>>(g, kind, a, b, X, Y); break;
-    }
-    EDAB_LAUNCH("riesz_spectrum");
+    launch_riesz<T>(s, g, kind, a, b, run, X, Y);
     const int odd = (kind == 0 || kind == 3) ? (1 << a) : (a == b ? 0 : ((1 << a) | (1 << b)));
     int kk[kMaxDim] = {1, 1, 1};
     for (int ax = 0; ax < D; ++ax) kk[ax] = ((odd >> ax) & 1) ? 2 : 1;
