@@ -173,6 +173,9 @@ namespace cg = cooperative_groups;
 constexpr int kDigitBits = 11;
 constexpr int kDigitBins = 1 << kDigitBits;
 constexpr int kSelClusterMax = 8;
+// Items of an element (at least, at most) and of the batch that the split form takes: its list of 8 % is
+// selected from by one CTA per element, which at 50 M items took 8.7 ms (the grid-wide form 2.9 ms).
+constexpr int64_t kSplitItems = 65536, kSplitMost = int64_t{1} << 22, kSplitTotal = int64_t{1} << 21;
 constexpr int kSelWide = 1024;  // threads of a cluster's CTA in a small batch
 // The cluster form for batches that fill the GPU with clusters (1), or the grid-wide form always (0).
 #ifndef EDAB_SEL_CLUSTERS
@@ -298,8 +301,8 @@ struct SelLeader {
 
 // The digit value of table tb (nb bins) that holds rank, and the rank inside it: one block-wide
 // exclusive prefix sum over the bins (nb / TH consecutive bins per thread, or one) of TH threads.
-template <int TH>
-__device__ __forceinline__ void rank_digit(const unsigned long long* tb, int nb, unsigned long long rank,
+template <int TH, class C>
+__device__ __forceinline__ void rank_digit(const C* tb, int nb, unsigned long long rank,
                                            unsigned long long* warp_tot, int* bin_out,
                                            unsigned long long* rest_out) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -635,6 +638,262 @@ __global__ void __launch_bounds__(kThreads) select_grid_pick(const int32_t* run,
   }
 }
 
+// The split form for many items (select): one pass over the items instead of one per digit. A sample of
+// the items brackets the statistic: the keys lo and hi of the sample about 5 standard deviations of
+// its rank to either side. The pass counts the items below lo and lists those in [lo, hi] (about 8 %);
+// when the wanted ranks lie in the list and it fits, a radix selection of the list is the answer, else
+// (a bracket that missed, or more ties than the list holds) the element is handed to the other forms.
+// Exact whatever the sample: the ranks are counted, not estimated. Bound by reading the items once
+// (a 512 x 512 element's median of differences: 230 us per 64 images before, the digit passes' counting).
+template <class K>
+struct SplitState {
+  K lo, hi;
+  unsigned long long less, total, listed;
+};
+static_assert(sizeof(SplitState<uint64_t>) <= sizeof(SelGridState<uint64_t>), "the split's states lie in the grid form's");
+
+constexpr int kSplitSample = 4096, kSplitThreads = 1024;
+
+template <class T, class K>
+__global__ void __launch_bounds__(kSplitThreads) split_pivots(Geom g, SelView<T> a, const int32_t* run, double q,
+                                                             SplitState<K>* st) {
+  __shared__ K keys[kSplitSample];
+  __shared__ int32_t found_s;
+  const int64_t b = blockIdx.x;
+  if (run && !run[b]) return;
+  if (threadIdx.x == 0) found_s = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < kSplitSample; i += kSplitThreads) {
+    // pseudo-random items (splitmix64 of the draw): a regular stride could fall in step with the field
+    uint64_t z = 0x9e3779b97f4a7c15ULL * static_cast<uint64_t>(i + 1);
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ULL;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebULL;
+    z ^= z >> 31;
+    const int64_t t = static_cast<int64_t>(__umul64hi(z, static_cast<uint64_t>(a.items)));
+    K k = K(0);
+    const bool have = sel_key_of<T, K>(g, a, b, t, &k);
+    keys[i] = have ? k : ~K(0);
+    const unsigned m = __ballot_sync(0xffffffffu, have);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&found_s, __popc(m));
+  }
+  for (int size = 2; size <= kSplitSample; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      __syncthreads();
+      for (int t = threadIdx.x; t < kSplitSample / 2; t += kSplitThreads) {
+        const int i = 2 * t - (t & (stride - 1)), j = i + stride;
+        const K x = keys[i], y = keys[j];
+        if ((x > y) == ((i & size) == 0)) {
+          keys[i] = y;
+          keys[j] = x;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int m = found_s;
+    const double rho = q < 0 ? 0.5 : q, at = rho * (m - 1);
+    const double spread = 5.0 * sqrt(rho * (1.0 - rho) * m) + 2.0;
+    const int lo = static_cast<int>(floor(at - spread)), hi = static_cast<int>(ceil(at + spread));
+    SplitState<K> s;
+    s.lo = lo < 0 ? K(0) : keys[lo];
+    s.hi = hi >= m ? ~K(0) : keys[hi];
+    s.less = s.total = s.listed = 0ULL;
+    st[b] = s;
+  }
+}
+
+// A warp's keys for the list, written 32 at a time.
+template <class K>
+__device__ __forceinline__ void list_keys(K* queue, int& held, bool listed, K key, const SelCand<K>& cand,
+                                          SplitState<K>* st, int64_t b) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = __ballot_sync(0xffffffffu, listed);
+  if (m == 0u) return;
+  if (listed) queue[held + __popc(m & ((1u << lane) - 1u))] = key;
+  held += __popc(m);
+  __syncwarp();
+  if (held >= 32) {
+    held -= 32;
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(&st[b].listed, 32ULL);
+    at = __shfl_sync(0xffffffffu, at, 0) + lane;
+    if (at < static_cast<unsigned long long>(cand.cap)) cand.keys[b * cand.cap + static_cast<int64_t>(at)] = queue[held + lane];
+    __syncwarp();
+  }
+}
+
+template <class T, class K>
+__global__ void __launch_bounds__(kThreads) split_count(Geom g, SelView<T> a, const int32_t* run, SplitState<K>* st,
+                                                       SelCand<K> cand) {
+  constexpr int W = 16 / static_cast<int>(sizeof(T));  // samples of a step of a thread: of one row
+  __shared__ K queue_s[kThreads / 32][64];
+  __shared__ unsigned long long less_s, total_s;
+  const int64_t b = blockIdx.y;
+  if (run && !run[b]) return;
+  if (threadIdx.x == 0) less_s = total_s = 0ULL;
+  __syncthreads();
+  const K lo = st[b].lo, hi = st[b].hi;
+  const bool diff = a.sel.src == SelSrc::kDiff;
+  const T* f = a.sel.field + b * g.field;
+  const uint8_t* mask = !diff && a.sel.mask ? a.sel.mask + b * g.field : nullptr;
+  const double center = a.sel.center ? a.sel.center[b] : 0.0;
+  const int32_t nl = elem_len(g, b);
+  const uint32_t units = static_cast<uint32_t>(g.field / W);  // per axis
+  K* queue = queue_s[threadIdx.x >> 5];
+  int held = 0;
+  uint32_t less = 0, total = 0;
+  const uint32_t step = gridDim.x * kThreads;
+  for (int ax = 0; ax < (diff ? a.naxes : 1); ++ax) {
+    const int axis = ax == 0 ? a.ax[0] : (ax == 1 ? a.ax[1] : a.ax[2]);
+    const bool last = axis == g.dim - 1;
+    const int64_t st_ax = last ? 1 : geom_stride(g, axis);
+    const int32_t n_ax = elem_n(g, b, axis);
+    for (uint32_t u = blockIdx.x * kThreads + threadIdx.x; u - (threadIdx.x & 31) < units; u += step) {
+      const int64_t v = static_cast<int64_t>(u) * W;
+      int32_t room = 0;  // samples of the step that are items
+      T x[W];
+      if (u < units) {
+        const int32_t col = static_cast<int32_t>(pitch_col(g, v));
+        room = min(W, nl - (diff && last ? 1 : 0) - col);
+        if (diff && !last && room > 0 && coord_of(g, v, axis) >= n_ax - 1) room = 0;
+        if (room > 0) {
+          const int4 p = *reinterpret_cast<const int4*>(f + v);
+          memcpy(x, &p, 16);
+          if (diff) {
+            T y[W];
+            if (last) {
+#pragma unroll
+              for (int k = 0; k + 1 < W; ++k) y[k] = x[k + 1];
+              y[W - 1] = room == W ? f[v + W] : T(0);
+            } else {
+              const int4 r = *reinterpret_cast<const int4*>(f + v + st_ax);
+              memcpy(y, &r, 16);
+            }
+#pragma unroll
+            for (int k = 0; k < W; ++k) x[k] = sub_rn(y[k], x[k]);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+        bool have = k < room;
+        if (have && mask) have = (mask[v + k] & a.sel.bits) != 0;
+        K key = K(0);
+        if constexpr (sizeof(K) == 4) {
+          key = order_key(static_cast<float>(x[k]));
+        } else {
+          double d = static_cast<double>(x[k]);
+          if (a.sel.center) d = fabs(__dsub_rn(d, center));
+          key = order_key(d);
+        }
+        total += have;
+        less += have && key < lo;
+        list_keys(queue, held, have && key >= lo && key <= hi, key, cand, st, b);
+      }
+    }
+  }
+  const int lane = threadIdx.x & 31;
+  if (held > 0) {
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(&st[b].listed, static_cast<unsigned long long>(held));
+    at = __shfl_sync(0xffffffffu, at, 0) + lane;
+    if (lane < held && at < static_cast<unsigned long long>(cand.cap)) cand.keys[b * cand.cap + static_cast<int64_t>(at)] = queue[lane];
+  }
+  less = __reduce_add_sync(0xffffffffu, less);
+  total = __reduce_add_sync(0xffffffffu, total);
+  if (lane == 0) {
+    atomicAdd(&less_s, static_cast<unsigned long long>(less));
+    atomicAdd(&total_s, static_cast<unsigned long long>(total));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (less_s) atomicAdd(&st[b].less, less_s);
+    if (total_s) atomicAdd(&st[b].total, total_s);
+  }
+}
+
+template <class K>
+__global__ void __launch_bounds__(kSplitThreads) split_finish(const int32_t* run, const SplitState<K>* st, SelCand<K> cand,
+                                                             double q, double* out, int64_t* count_out, int32_t* mask) {
+  constexpr int kKeyBits = 8 * static_cast<int>(sizeof(K));
+  constexpr int kDigits = (kKeyBits + kDigitBits - 1) / kDigitBits;
+  __shared__ uint32_t local[2 * kDigitBins];
+  __shared__ unsigned long long warp_tot[kSplitThreads / 32];
+  __shared__ int hit_bin;
+  __shared__ unsigned long long hit_rest;
+  const int64_t b = blockIdx.x;
+  const int tid = threadIdx.x;
+  if (run && !run[b]) {
+    if (tid == 0) mask[b] = 0;
+    return;
+  }
+  const SplitState<K> s = st[b];
+  unsigned long long rank[2] = {0, 0};
+  double gamma = 0.0;
+  if (s.total > 0) {
+    if (q < 0) {
+      rank[0] = (s.total - 1) / 2;
+      rank[1] = s.total / 2;
+    } else {
+      long long i = 0, j = 0;
+      linear_index(static_cast<long long>(s.total), q, &i, &j, &gamma);
+      rank[0] = static_cast<unsigned long long>(i);
+      rank[1] = static_cast<unsigned long long>(j);
+    }
+  }
+  const bool tie = s.lo == s.hi;  // every listed key is the same
+  const bool ok = s.total == 0 || (rank[0] >= s.less && rank[1] < s.less + s.listed &&
+                                   (tie || s.listed <= static_cast<unsigned long long>(cand.cap)));
+  if (tid == 0) mask[b] = ok ? 0 : 1;
+  if (!ok) return;
+  if (s.total == 0) {
+    if (tid == 0) {
+      out[b] = d_nan();
+      if (count_out) count_out[b] = 0;
+    }
+    return;
+  }
+  K prefix[2] = {K(0), K(0)};
+  if (tie) {
+    prefix[0] = prefix[1] = s.lo;
+  } else {
+    rank[0] -= s.less;
+    rank[1] -= s.less;
+    const K* keys = cand.keys + b * cand.cap;
+    const int64_t n = static_cast<int64_t>(s.listed);
+    for (int pass = 0; pass < kDigits; ++pass) {
+      int hi, shift, width;
+      digit_of_pass<kKeyBits>(pass, &hi, &shift, &width);
+      const K dmask = static_cast<K>((K(1) << width) - K(1));
+      const bool two = pass > 0 && prefix[0] != prefix[1];
+      for (int i = tid; i < 2 * kDigitBins; i += kSplitThreads) local[i] = 0u;
+      __syncthreads();
+      for (int64_t t = tid; t - (tid & 31) < n; t += kSplitThreads) {
+        const bool have = t < n;
+        const K k = have ? keys[t] : K(0);
+        const uint32_t digit = static_cast<uint32_t>((k >> shift) & dmask);
+        const K top = pass == 0 ? K(0) : (k >> hi);
+        count_digit(local, digit, have && (pass == 0 || top == (prefix[0] >> hi)));
+        if (two) count_digit(local + kDigitBins, digit, have && top == (prefix[1] >> hi));
+      }
+      __syncthreads();
+      const int bins = 1 << width;
+      for (int r = 0; r < 2; ++r) {
+        rank_digit<kSplitThreads>(local + (two ? r : 0) * kDigitBins, bins, rank[r], warp_tot, &hit_bin, &hit_rest);
+        prefix[r] |= static_cast<K>(hit_bin) << shift;
+        rank[r] = hit_rest;
+        __syncthreads();
+      }
+    }
+  }
+  if (tid == 0) {
+    const double v0 = key_value(prefix[0]), v1 = key_value(prefix[1]);
+    out[b] = q < 0 ? ((s.total & 1) ? v0 : __dmul_rn(__dadd_rn(v0, v1), 0.5)) : linear_between(v0, v1, gamma);
+    if (count_out) count_out[b] = static_cast<int64_t>(s.total);
+  }
+}
+
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 }  // namespace
@@ -657,6 +916,7 @@ void field_totals(cudaStream_t s, const Geom& g, const T* f, double* energy, dou
   EDAB_LAUNCH("element_totals");
 }
 
+constexpr int64_t kMaskKeys = 32;
 // Candidate keys per element: a quarter of the largest selection's items (the differences along
 // every axis), at least 64.
 int64_t cand_cap(const Geom& g) { return std::max<int64_t>(64, static_cast<int64_t>(g.dim) * g.field / 4 / 32 * 32); }
@@ -676,8 +936,14 @@ SelCand<K> cand_of(const Geom& g, void* scratch) {
   SelCand<K> c;
   c.n = reinterpret_cast<unsigned long long*>(p);
   c.keys = reinterpret_cast<K*>(p + align256(B * sizeof(unsigned long long)));
-  c.cap = cand_cap(g);
+  c.cap = cand_cap(g) - kMaskKeys;
   return c;
+}
+// The split selection's run mask of the elements that it hands on, behind the candidate lists (each of
+// which is kMaskKeys shorter than its share of the scratch).
+template <class K>
+int32_t* split_mask(const Geom& g, const SelCand<K>& c) {
+  return reinterpret_cast<int32_t*>(c.keys + static_cast<size_t>(g.batch) * c.cap);
 }
 
 // The grid-wide form: every digit a counting and a pick launch (scratch: the states, then the
@@ -707,6 +973,26 @@ void select_grid(cudaStream_t s, const Geom& g, const SelView<T>& a, double q, c
   }
 }
 
+// The split form of a selection; returns the run mask of the elements that it hands on.
+template <class T, class K>
+const int32_t* select_split(cudaStream_t s, const Geom& g, const SelView<T>& a, double q, const int32_t* run, double* out,
+                            int64_t* count, void* scratch, int sms) {
+  const SelCand<K> cand = cand_of<K>(g, scratch);
+  auto* st = static_cast<SplitState<K>*>(scratch);
+  int32_t* mask = split_mask(g, cand);
+  const unsigned B = static_cast<unsigned>(g.batch);
+  split_pivots<T, K><<<B, kSplitThreads, 0, s>>>(g, a, run, q, st);
+  EDAB_LAUNCH("split_pivots");
+  // 8 CTAs per SM in all, at least 16 items per thread
+  const int64_t fill = (int64_t{8} * sms + g.batch - 1) / g.batch;
+  const unsigned ctas = static_cast<unsigned>(std::clamp<int64_t>(fill, 1, std::max<int64_t>(1, a.items / (int64_t{kThreads} * 16))));
+  split_count<T, K><<<dim3(ctas, B), kThreads, 0, s>>>(g, a, run, st, cand);
+  EDAB_LAUNCH("split_count");
+  split_finish<K><<<B, kSplitThreads, 0, s>>>(run, st, cand, q, out, count, mask);
+  EDAB_LAUNCH("split_finish");
+  return mask;
+}
+
 template <class T>
 void select(cudaStream_t s, const Geom& g, const Sel<T>& sel, double q, const int32_t* run, double* out,
             int64_t* count, void* scratch) {
@@ -732,6 +1018,17 @@ void select(cudaStream_t s, const Geom& g, const Sel<T>& sel, double q, const in
     int dev = 0;
     EDAB_CUDA(cudaGetDevice(&dev));
     EDAB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  }
+  // Many items: the split form first, then the others for the elements that it hands on.
+  if (scratch && a.items >= kSplitItems && a.items <= kSplitMost && a.items * g.batch >= kSplitTotal) {
+    bool done = false;
+    if constexpr (std::is_same_v<T, float>) {
+      if (sel.center == nullptr) {
+        run = select_split<T, uint32_t>(s, g, a, q, run, out, count, scratch, sms);
+        done = true;
+      }
+    }
+    if (!done) run = select_split<T, uint64_t>(s, g, a, q, run, out, count, scratch, sms);
   }
   const bool many = g.batch * kSelClusterMax >= 2 * static_cast<int64_t>(sms);
   if (!kSelClusters || (!many && a.items > int64_t{kSelClusterMax} * kSelWide * 8)) {
