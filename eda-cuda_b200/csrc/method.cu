@@ -200,6 +200,17 @@ __device__ __forceinline__ T times_pow2(T v, int32_t k) {
   else return ldexp(v, k);
 }
 
+// A row's value v with the element's prescale undone; a value that leaves the dtype's range fails the
+// element. (Applied as the rows are written: a pass of its own over every row that a call may have
+// took 0.6 ms per 64 images of 512 x 512.)
+template <class T>
+__device__ __forceinline__ T unscaled(Elem& e, T v) {
+  if (e.exp == 0) return v;
+  const T y = times_pow2(v, e.exp);
+  if (!isfinite(y)) e.error = kErrNonFiniteResult;
+  return y;
+}
+
 template <class T>
 __device__ __forceinline__ double tie_tol(double tau, double amax) {
   return static_cast<double>(mul_rn(static_cast<T>(tau), static_cast<T>(amax)));
@@ -1337,7 +1348,7 @@ bool Engine<T>::commit() {
                const int64_t q = pitch_row(g, v);
                const int64_t t = v - q * g.pitch;
                const T hv = h[i];
-               rows[(b * c.rows_cap + el[b].n_imfs) * g.count + q * nl + t] = hv;
+               rows[(b * c.rows_cap + el[b].n_imfs) * g.count + q * nl + t] = unscaled(el[b], hv);
                r[i] = sub_rn(r[i], hv);
              });
   double* eh = dsc_ + 0 * B_;
@@ -1605,7 +1616,7 @@ void Engine<T>::run(const T* x, T* rows_out, int32_t* hist_scale, int32_t* hist_
     std::swap(L_, Lp_);
     if (!more) break;
   }
-  // finish: the residue row, the rows scaled back
+  // finish: the residue row
   {
     const int32_t nl2 = g_.n_last;
     T* rows = rows_;
@@ -1613,20 +1624,8 @@ void Engine<T>::run(const T* x, T* rows_out, int32_t* hist_scale, int32_t* hist_
                [=] __device__(int64_t b, int64_t v, int64_t i) {
                  const int64_t q = pitch_row(g, v);
                  const int64_t t = v - q * g.pitch;
-                 rows[(b * c.rows_cap + el[b].n_imfs) * g.count + q * nl2 + t] = r[i];
+                 rows[(b * c.rows_cap + el[b].n_imfs) * g.count + q * nl2 + t] = unscaled(el[b], r[i]);
                });
-    const int64_t per = static_cast<int64_t>(c.rows_cap) * g.count;
-    for_samples(s_, B_ * per, [=] __device__(int64_t idx) {
-      const int64_t b = idx / per;
-      const int32_t k = el[b].exp;
-      if (k == 0 || el[b].status == kError) return;
-      const int64_t at = idx - b * per;
-      if (at / g.count > el[b].n_imfs) return;
-      if (g.len && at % g.count >= elem_len(g, b)) return;  // beyond the element's length: never written
-      const T v = times_pow2(rows[idx], k);
-      rows[idx] = v;
-      if (!isfinite(v)) el[b].error = kErrNonFiniteResult;
-    });
   }
   out.resize(static_cast<size_t>(B_));
   EDAB_CUDA(cudaMemcpyAsync(out.data(), el_, sizeof(Elem) * B_, cudaMemcpyDeviceToHost, s_));
