@@ -58,11 +58,15 @@ struct StepTree {
 };
 
 // One step of a row: the warp's tree over the chunks [32 step, 32 step + 32), staged by coalesced loads
-// (a chunk per lane read straight from global memory took 73 us per 64 images of 512 x 512, a load
-// per lane and sample); the lane's max |v| and non-finite samples are added to amax and bad.
+// and padded with zeros (+0 changes no sum of squares); the lane's max |v| (as T's bits) and whether a
+// sample is not finite are added to amax and bad (counted).
 template <class T>
-__device__ __forceinline__ double row_step(const T* __restrict__ row, int32_t n, int32_t step, T* tile, uint64_t& amax,
+using BitsOf = std::conditional_t<sizeof(T) == 4, uint32_t, uint64_t>;
+template <class T>
+__device__ __forceinline__ double row_step(const T* __restrict__ row, int32_t n, int32_t step, T* tile, BitsOf<T>& amax,
                                            unsigned& bad) {
+  using U = BitsOf<T>;
+  constexpr U kAbs = ~U(0) >> 1, kInf = sizeof(T) == 4 ? U(0x7f800000u) : static_cast<U>(0x7ff0000000000000ULL);
   const int lane = threadIdx.x & 31;
   const int32_t i0 = step * 1024, left = min(n - i0, 1024);
   __syncwarp();
@@ -73,14 +77,24 @@ __device__ __forceinline__ double row_step(const T* __restrict__ row, int32_t n,
   }
   __syncwarp();
   double acc = 0.0;
-  const int32_t len = min(32, left - 32 * lane);
-  for (int32_t j = 0; j < len; ++j) {
-    const T v = tile[33 * lane + j];
-    const double d = static_cast<double>(v);
-    acc = __dadd_rn(acc, __dmul_rn(d, d));
-    const uint64_t ab = abs_bits(v);
-    amax = ab > amax ? ab : amax;
-    bad += isfinite(d) ? 0u : 1u;
+  if (32 * lane < left) {
+    const T* t = tile + 33 * lane;
+#pragma unroll 2
+    for (int32_t j = 0; j < 32; j += 8) {
+      T v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = t[j + k];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const double d = static_cast<double>(v[k]);
+        acc = __dadd_rn(acc, __dmul_rn(d, d));
+        U u;
+        memcpy(&u, &v[k], sizeof u);
+        u &= kAbs;
+        amax = max(amax, u);
+        bad += u >= kInf ? 1u : 0u;
+      }
+    }
   }
   return warp_tree32(acc);
 }
@@ -95,7 +109,7 @@ __global__ void __launch_bounds__(kRowThreads<T>) row_partials(const T* __restri
                                                          uint64_t* nonfinite, bool per_row) {
   __shared__ T tile_s[kRowThreads<T> / 32][32 * 33];
   __shared__ double step_s[kMaxSteps];
-  __shared__ uint64_t amax_s[kRowThreads<T> / 32];
+  __shared__ BitsOf<T> amax_s[kRowThreads<T> / 32];
   __shared__ unsigned bad_s[kRowThreads<T> / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t total = g.batch * g.rows;
@@ -105,7 +119,7 @@ __global__ void __launch_bounds__(kRowThreads<T>) row_partials(const T* __restri
     const int32_t n = g.len ? elem_len(g, q / g.rows) : g.n_last;
     const int32_t steps = (n + 1023) >> 10;
     const T* row = f + q * g.pitch;
-    uint64_t amax = 0;
+    BitsOf<T> amax = 0;
     unsigned bad = 0;
     double one = 0.0;
     for (int32_t k = per_row ? warp : 0; k < steps; k += kRowThreads<T> / 32) {
@@ -114,7 +128,7 @@ __global__ void __launch_bounds__(kRowThreads<T>) row_partials(const T* __restri
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
-      const uint64_t o = __shfl_down_sync(0xffffffffu, amax, d);
+      const BitsOf<T> o = __shfl_down_sync(0xffffffffu, amax, d);
       amax = o > amax ? o : amax;
       bad += __shfl_down_sync(0xffffffffu, bad, d);
     }
@@ -135,7 +149,9 @@ __global__ void __launch_bounds__(kRowThreads<T>) row_partials(const T* __restri
       }
     }
     if (per_row ? threadIdx.x == 0 : lane == 0) {
-      rows[q] = RowPartial{one, amax};
+      T largest;
+      memcpy(&largest, &amax, sizeof largest);
+      rows[q] = RowPartial{one, abs_bits(largest)};
       if (nonfinite && bad) atomicAdd(reinterpret_cast<unsigned long long*>(&nonfinite[q / g.rows]), bad);
     }
     if (per_row) __syncthreads();  // the next row rewrites the steps' sums
