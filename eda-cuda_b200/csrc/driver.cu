@@ -23,6 +23,7 @@ void Workspace::release() {
     int prev = -1;
     cudaGetDevice(&prev);
     if (device_ >= 0 && prev != device_) cudaSetDevice(device_);
+    replays_.clear();
     cudaFree(base_);
     if (device_ >= 0 && prev != device_ && prev >= 0) cudaSetDevice(prev);
   }
@@ -61,7 +62,9 @@ std::vector<std::unique_ptr<Workspace>>& idle_workspaces() {
 
 Workspace& thread_workspace() {
   thread_local Workspace ws;
-  return t_leased ? *t_leased : ws;
+  if (t_leased) return *t_leased;
+  ws.keep_replays();
+  return ws;
 }
 
 void set_thread_workspace(Workspace* ws) { t_leased = ws; }

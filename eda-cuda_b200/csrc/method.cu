@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdio>
 #include <set>
+#include <string>
 #include <vector>
 
 namespace edab {
@@ -575,6 +576,9 @@ class Engine {
   Engine(const Geom& g, const Ctl& c, cudaStream_t s, Workspace& ws) : g_(g), c_(c), s_(s) { bind(ws); }
   // return_orientation: rows (B, rows_cap - 1, D + 1, count) receiving n and c of every mode
   T* orient_out_ = nullptr;
+  // the replayed launch sequences (nullptr: every launch is issued)
+  Replays* replays_ = nullptr;
+  const void* base_ = nullptr;  // the workspace
 
   // x: the chunk's input, dense (B, count) on the device. Rows into rows_out (B, cap, count).
   void run(const T* x, T* rows_out, int32_t* hist_scale, int32_t* hist_sifts, double* hist_spacing,
@@ -619,17 +623,49 @@ class Engine {
   }
   void write_el() { EDAB_CUDA(cudaMemcpyAsync(el_, hel_.data(), sizeof(Elem) * B_, cudaMemcpyHostToDevice, s_)); }
 
+  // Issues the launches of `body` (sequence `part` of a mode, which depends on nothing but the engine's
+  // geometry, constants and buffers and on `count`), or replays them.
+  template <class F>
+  void sequence(int part, int32_t count, F body) {
+    if (!replays_) {
+      body();
+      return;
+    }
+    std::string key;
+    const auto put = [&](const auto& v) { key.append(reinterpret_cast<const char*>(&v), sizeof v); };
+    const CubeTune tune = cube_tune_for(g_, 0, sizeof(T));
+    const int32_t ints[] = {part, count, static_cast<int32_t>(sizeof(T)), g_.dim, g_.n[0], g_.n[1], g_.n[2],
+                            static_cast<int32_t>(transform_precision()), tune.lines, c_.sifts, c_.check_finite, c_.max_imf, c_.rows_cap};
+    put(ints);
+    put(g_.batch);
+    put(c_.tau);
+    put(base_);
+    put(L_);
+    replays_->run(key, s_, [&](cudaStream_t s) {
+      struct Stream {  // the engine's stream again, also after an error
+        cudaStream_t& at;
+        cudaStream_t kept;
+        ~Stream() { at = kept; }
+      } back{s_, s_};
+      s_ = s;
+      body();
+    });
+  }
   void noise(const T* r, unsigned axes, const int32_t* run, double* out);
   void noise_per_axis(const T* r, const int32_t* run, double* out);
   void tau_field(const int32_t* run, bool floor2, T* tau);
   void raw_window(const uint8_t* flags, const int32_t* w, const int32_t* run, T* om, T* tmp);
   void scale_field();
   void local_floor();
-  void g2();
+  int32_t g2_candidates(bool* active);
+  void g2(int32_t steps);
+  void mode_start();
+  void element_fields();
   void g2_test(const uint8_t* ff, uint8_t* P);
   void orientation_and_build();
   void store_orientation();
-  bool ladder_and_weights(int32_t* n_rungs_max);
+  bool ladders(int32_t* n_rungs_max);
+  void weights(int32_t n_rungs_max);
   void op(int which, const T* in, const GatherOut<T>& out, int32_t n_rungs_max);
   void envelope_mean(const T* h, const GatherOut<T>& ext, const GatherOut<T>& mean, int32_t nrm);
   void sifts(int32_t nrm);
@@ -918,17 +954,20 @@ void Engine<T>::g2_test(const uint8_t* ff, uint8_t* P) {
 }
 
 // G2 and G3 (cpp/src/method/driver.cpp:445-509; the machine of driver.cpp:73-116 on the device).
+// S1: the candidates of every G2-eligible element (host pow). Returns the rung tests to run (0: no element
+// has a candidate) and whether any element is active.
 template <class T>
-void Engine<T>::g2() {
-  // S1: the candidates of every G2-eligible element (host pow)
+int32_t Engine<T>::g2_candidates(bool* active) {
   read_el();
   int32_t steps = 0;
   bool any = false;
+  *active = false;
   for (int64_t b = 0; b < B_; ++b) {
     Elem& e = hel_[static_cast<size_t>(b)];
     e.g2_n = 0;
     e.g2_done = 1;
     e.g2_accepted = 0;
+    *active = *active || e.status == kActive;
     if (e.status != kActive || !e.on_g2) continue;
     const std::vector<int32_t> rungs = g2_candidate_rungs(e.w, e.w_prev, c_.fine_jump);
     e.g2_n = static_cast<int32_t>(rungs.size());
@@ -942,7 +981,12 @@ void Engine<T>::g2() {
     any = any || !rungs.empty();
   }
   write_el();
-  if (!any) return;
+  return any ? steps : 0;
+}
+
+template <class T>
+void Engine<T>::g2(int32_t steps) {
+  if (steps == 0) return;
   Elem* el = el_;
   int32_t* ong2 = mask(kOnG2);
   for_elements(s_, B_, [=] __device__(int64_t b) { ong2[b] = el[b].status == kActive && el[b].on_g2; });
@@ -1062,7 +1106,6 @@ void Engine<T>::orientation_and_build() {
     for_elements(s_, B_, [=] __device__(int64_t b) {
       if (el[b].status == kActive && el[b].nonfinite) fail2(el[b], win_s, mask_s, B, b);
     });
-    if (orient_out_) store_orientation();
   }
   const dim3 grid = voxel_grid(g_);
   switch (g_.dim) {
@@ -1102,9 +1145,9 @@ void Engine<T>::store_orientation() {
              });
 }
 
-// S4: the ladders (host), then the rung logs, the weights and the rung windows.
+// S4: the ladders (host); false when no element is active.
 template <class T>
-bool Engine<T>::ladder_and_weights(int32_t* n_rungs_max) {
+bool Engine<T>::ladders(int32_t* n_rungs_max) {
   read_el();
   int32_t nrm = 0;
   bool any = false;
@@ -1129,7 +1172,12 @@ bool Engine<T>::ladder_and_weights(int32_t* n_rungs_max) {
   }
   write_el();
   *n_rungs_max = nrm;
-  if (!any) return false;
+  return any;
+}
+
+// The rung logs, the weights and the rung windows.
+template <class T>
+void Engine<T>::weights(int32_t nrm) {
   Elem* el = el_;
   const int32_t* on = mask(kOn);
   for_samples(s_, B_ * kMaxRungs, [=] __device__(int64_t i) {
@@ -1148,7 +1196,6 @@ bool Engine<T>::ladder_and_weights(int32_t* n_rungs_max) {
     const bool use = e.status == kActive && j < nrm && j < e.n_rungs && ((e.rung_used >> j) & 1u) != 0u;
     rw[i] = use ? e.rung_w[j] : 0;
   });
-  return true;
 }
 
 // An operator over every used rung: the rung cubes (one launch per pass for all rungs; the first
@@ -1396,6 +1443,167 @@ bool Engine<T>::commit() {
   return flags[0] != 0;
 }
 
+// Steps 0-2 of a mode: its state and noise level, the window passes.
+template <class T>
+void Engine<T>::mode_start() {
+  const Ctl c = c_;
+  const Geom g = g_;
+  const int64_t B = B_;
+  Elem* el = el_;
+  int32_t* winp = win_;
+  int32_t* maskp = mask_;
+  // step 0: mode start (cpp/src/method/mode.cu:95-136)
+  for_elements(s_, B_, [=] __device__(int64_t b) {
+    Elem& e = el[b];
+    if (e.status != kActive) {
+      leave(e, winp, maskp, B, b, e.status);
+      return;
+    }
+    e.r_inf = e.amax;
+    for (int a = 0; a < kMaxDim; ++a) e.ext[a] = 0;
+    e.fine = 0;
+    e.jump = c.absent_jump;
+    e.p_odd = 0;
+    e.p = 0.0;
+    e.cov = 0.0;
+    e.wc = d_inf();
+    e.g3 = 1.0;
+    e.sifting = 1;
+    e.n_sifts = 0;
+    e.gmax_res_bits = 0;
+    e.gmax_h_bits = 0;
+    e.on_g2 = 0;
+    const int32_t w0 = max(3, e.w_prev + 2);
+    int32_t wd, wl;
+    tau_windows(c, w0, &wd, &wl);
+    for (int k = 0; k < kSlots; ++k) winp[k * B + b] = 0;
+    winp[kWd * B + b] = wd;
+    winp[kWl * B + b] = wl;
+    maskp[kOn * B + b] = 1;
+    maskp[kOnG2 * B + b] = 0;
+    maskp[kOnFloor * B + b] = e.k >= 1 ? 1 : 0;
+    maskp[kOnFine * B + b] = 0;
+  });
+  noise(r_, (1u << g_.dim) - 1u, mask(kOn), dsc_ + 7 * B_);
+  {
+    const double* sn = dsc_ + 7 * B_;
+    const int32_t* on = mask(kOn);
+    for_elements(s_, B_, [=] __device__(int64_t b) {
+      if (on[b]) el[b].sigma_n = sn[b];
+    });
+  }
+  // steps 1-2: the window passes
+  for (int32_t pass = 0; pass < c_.sig_passes; ++pass) {
+    tau_field(mask(kOn), false, tau_);
+    for_elements(s_, B_, [=] __device__(int64_t b) {
+      if (el[b].status == kActive && el[b].nonfinite) fail2(el[b], winp, maskp, B, b);
+    });
+    sig_flags<T>(s_, g_, r_, tau_, flags_, el_, mask(kOn));
+    const int32_t ps = pass;
+    for_elements(s_, B_, [=] __device__(int64_t b) {
+      Elem& e = el[b];
+      if (e.status != kActive) return;
+      const uint64_t N = static_cast<uint64_t>(elem_count(g, b));
+      uint64_t S2 = 0;
+      bool enough = false;
+      for (int a = 0; a < g.dim; ++a) {
+        const uint64_t ea = e.ext[a];
+        S2 += ea * ea;
+        if (ea * static_cast<uint64_t>(elem_n(g, b, a)) >= 3 * N) enough = true;
+      }
+      for (int a = 0; a < kMaxDim; ++a) e.ext[a] = 0;
+      if (!enough) {
+        leave(e, winp, maskp, B, b, kDone);
+        return;
+      }
+      const double sp = __ddiv_rn(static_cast<double>(N), __dsqrt_rn(static_cast<double>(S2)));
+      const double v = __dmul_rn(__dmul_rn(2.0, c.kappa), sp);
+      if (!(v < 1073741824.0)) {
+        leave(e, winp, maskp, B, b, kDone);
+        return;
+      }
+      int32_t w = 2 * static_cast<int32_t>(floor((v > 1.0 ? v : 1.0) / 2.0)) + 1;
+      w = max(w, 3);
+      w = max(w, e.w_prev + 2);
+      if (w > (g.len ? elem_len(g, b) : c.n_max)) {
+        leave(e, winp, maskp, B, b, kDone);
+        return;
+      }
+      e.spacing = sp;
+      int32_t wd, wl;
+      tau_windows(c, w, &wd, &wl);
+      winp[kWd * B + b] = wd;
+      winp[kWl * B + b] = wl;
+      if (ps == c.sig_passes - 1) {
+        e.w = w;
+        const int32_t s0 = max(3, e.w_prev + 2);
+        e.on_g2 = (__dmul_rn(c.fine_jump, static_cast<double>(s0)) <= static_cast<double>(w)) ? 1 : 0;
+      }
+    });
+  }
+}
+
+// Steps 4-6 of a mode: the window, the scale field, the orientation and the element's extent.
+template <class T>
+void Engine<T>::element_fields() {
+  const Ctl c = c_;
+  const Geom g = g_;
+  const int64_t B = B_;
+  Elem* el = el_;
+  int32_t* winp = win_;
+  int32_t* maskp = mask_;
+  // step 4: the guard, the window (cpp/src/method/mode.cu:189-223)
+  for_elements(s_, B_, [=] __device__(int64_t b) {
+    Elem& e = el[b];
+    if (e.status == kActive && e.nonfinite) {
+      fail2(e, winp, maskp, B, b);
+      return;
+    }
+    if (e.status != kActive) return;
+    int32_t w = e.w;
+    if (e.fine) {
+      w = max(max(e.p_odd, e.w_prev + 2), 3);
+      e.jump = 1.0;
+    }
+    if (c.growth > 1.0 && e.k >= c.growth_from) {
+      w = max(w, odd_window(__dmul_rn(c.growth, static_cast<double>(e.w_prev))));
+      if (w > (g.len ? elem_len(g, b) : c.n_max)) {
+        leave(e, winp, maskp, B, b, kDone);
+        return;
+      }
+    }
+    e.w = w;
+    const int32_t W = odd_window(__dmul_rn(c.beta, static_cast<double>(w)));
+    e.W = W;
+    winp[kW * B + b] = W;
+    if (e.fine) {
+      double f = 1.0;
+      if (isfinite(e.wc)) {
+        const double qq = __dsqrt_rn(__ddiv_rn(e.wc, static_cast<double>(e.p_odd)));
+        f = __ddiv_rn(__dmul_rn(c.split, qq), 2.0);
+        f = f < 1.0 ? f : 1.0;
+      }
+      e.g3 = f;
+    }
+    e.d_min_bits = 0x7ff0000000000000ULL;
+    e.d_max_bits = 0;
+  });
+  // step 5: the scale field, the floor, G3's scaling
+  raw_window(flags_, win(kW), mask(kOn), om_, tmp_);
+  scale_field();
+  local_floor();
+  {
+    T* L = L_;
+    for_voxels(s_, g_, [=] __device__(int64_t b) { return el[b].status == kActive && el[b].fine; },
+               [=] __device__(int64_t b, int64_t, int64_t i) {
+                 const T v = mul_rn(static_cast<T>(el[b].g3), L[i]);
+                 L[i] = v >= T(3) ? v : T(3);
+               });
+  }
+  // step 6: orientation and the element build
+  orientation_and_build();
+}
+
 template <class T>
 void Engine<T>::run(const T* x, T* rows_out, int32_t* hist_scale, int32_t* hist_sifts, double* hist_spacing,
                     double* hist_energy, std::vector<Elem>& out) {
@@ -1462,155 +1670,24 @@ void Engine<T>::run(const T* x, T* rows_out, int32_t* hist_scale, int32_t* hist_
   EDAB_CUDA(cudaMemsetAsync(Lp_, 0, sizeof(T) * B_ * g_.field, s_));
 
   for (;;) {
-    // step 0: mode start (cpp/src/method/mode.cu:95-136)
-    for_elements(s_, B_, [=] __device__(int64_t b) {
-      Elem& e = el[b];
-      if (e.status != kActive) {
-        leave(e, winp, maskp, B, b, e.status);
-        return;
-      }
-      e.r_inf = e.amax;
-      for (int a = 0; a < kMaxDim; ++a) e.ext[a] = 0;
-      e.fine = 0;
-      e.jump = c.absent_jump;
-      e.p_odd = 0;
-      e.p = 0.0;
-      e.cov = 0.0;
-      e.wc = d_inf();
-      e.g3 = 1.0;
-      e.sifting = 1;
-      e.n_sifts = 0;
-      e.gmax_res_bits = 0;
-      e.gmax_h_bits = 0;
-      e.on_g2 = 0;
-      const int32_t w0 = max(3, e.w_prev + 2);
-      int32_t wd, wl;
-      tau_windows(c, w0, &wd, &wl);
-      for (int k = 0; k < kSlots; ++k) winp[k * B + b] = 0;
-      winp[kWd * B + b] = wd;
-      winp[kWl * B + b] = wl;
-      maskp[kOn * B + b] = 1;
-      maskp[kOnG2 * B + b] = 0;
-      maskp[kOnFloor * B + b] = e.k >= 1 ? 1 : 0;
-      maskp[kOnFine * B + b] = 0;
+    // steps 0-2
+    sequence(0, 0, [&] { mode_start(); });
+    // step 3: G2's candidates (S1), then its rung tests; steps 4-6
+    bool active = false;
+    const int32_t steps = g2_candidates(&active);
+    if (!active) break;
+    sequence(1, steps, [&] {
+      g2(steps);
+      element_fields();
     });
-    noise(r_, (1u << g_.dim) - 1u, mask(kOn), dsc_ + 7 * B_);
-    {
-      const double* sn = dsc_ + 7 * B_;
-      const int32_t* on = mask(kOn);
-      for_elements(s_, B_, [=] __device__(int64_t b) {
-        if (on[b]) el[b].sigma_n = sn[b];
-      });
-    }
-    // steps 1-2: the window passes
-    for (int32_t pass = 0; pass < c_.sig_passes; ++pass) {
-      tau_field(mask(kOn), false, tau_);
-      for_elements(s_, B_, [=] __device__(int64_t b) {
-        if (el[b].status == kActive && el[b].nonfinite) fail2(el[b], winp, maskp, B, b);
-      });
-      sig_flags<T>(s_, g_, r_, tau_, flags_, el_, mask(kOn));
-      const int32_t ps = pass;
-      for_elements(s_, B_, [=] __device__(int64_t b) {
-        Elem& e = el[b];
-        if (e.status != kActive) return;
-        const uint64_t N = static_cast<uint64_t>(elem_count(g, b));
-        uint64_t S2 = 0;
-        bool enough = false;
-        for (int a = 0; a < g.dim; ++a) {
-          const uint64_t ea = e.ext[a];
-          S2 += ea * ea;
-          if (ea * static_cast<uint64_t>(elem_n(g, b, a)) >= 3 * N) enough = true;
-        }
-        for (int a = 0; a < kMaxDim; ++a) e.ext[a] = 0;
-        if (!enough) {
-          leave(e, winp, maskp, B, b, kDone);
-          return;
-        }
-        const double sp = __ddiv_rn(static_cast<double>(N), __dsqrt_rn(static_cast<double>(S2)));
-        const double v = __dmul_rn(__dmul_rn(2.0, c.kappa), sp);
-        if (!(v < 1073741824.0)) {
-          leave(e, winp, maskp, B, b, kDone);
-          return;
-        }
-        int32_t w = 2 * static_cast<int32_t>(floor((v > 1.0 ? v : 1.0) / 2.0)) + 1;
-        w = max(w, 3);
-        w = max(w, e.w_prev + 2);
-        if (w > (g.len ? elem_len(g, b) : c.n_max)) {
-          leave(e, winp, maskp, B, b, kDone);
-          return;
-        }
-        e.spacing = sp;
-        int32_t wd, wl;
-        tau_windows(c, w, &wd, &wl);
-        winp[kWd * B + b] = wd;
-        winp[kWl * B + b] = wl;
-        if (ps == c.sig_passes - 1) {
-          e.w = w;
-          const int32_t s0 = max(3, e.w_prev + 2);
-          e.on_g2 = (__dmul_rn(c.fine_jump, static_cast<double>(s0)) <= static_cast<double>(w)) ? 1 : 0;
-        }
-      });
-    }
-    // step 3: G2 (S1 inside)
-    g2();
-    bool any_active = false;
-    for (const Elem& e : hel_) any_active = any_active || e.status == kActive;
-    if (!any_active) break;
-    // step 4: the guard, the window (cpp/src/method/mode.cu:189-223)
-    for_elements(s_, B_, [=] __device__(int64_t b) {
-      Elem& e = el[b];
-      if (e.status == kActive && e.nonfinite) {
-        fail2(e, winp, maskp, B, b);
-        return;
-      }
-      if (e.status != kActive) return;
-      int32_t w = e.w;
-      if (e.fine) {
-        w = max(max(e.p_odd, e.w_prev + 2), 3);
-        e.jump = 1.0;
-      }
-      if (c.growth > 1.0 && e.k >= c.growth_from) {
-        w = max(w, odd_window(__dmul_rn(c.growth, static_cast<double>(e.w_prev))));
-        if (w > (g.len ? elem_len(g, b) : c.n_max)) {
-          leave(e, winp, maskp, B, b, kDone);
-          return;
-        }
-      }
-      e.w = w;
-      const int32_t W = odd_window(__dmul_rn(c.beta, static_cast<double>(w)));
-      e.W = W;
-      winp[kW * B + b] = W;
-      if (e.fine) {
-        double f = 1.0;
-        if (isfinite(e.wc)) {
-          const double qq = __dsqrt_rn(__ddiv_rn(e.wc, static_cast<double>(e.p_odd)));
-          f = __ddiv_rn(__dmul_rn(c.split, qq), 2.0);
-          f = f < 1.0 ? f : 1.0;
-        }
-        e.g3 = f;
-      }
-      e.d_min_bits = 0x7ff0000000000000ULL;
-      e.d_max_bits = 0;
-    });
-    // step 5: the scale field, the floor, G3's scaling
-    raw_window(flags_, win(kW), mask(kOn), om_, tmp_);
-    scale_field();
-    local_floor();
-    {
-      T* L = L_;
-      for_voxels(s_, g_, [=] __device__(int64_t b) { return el[b].status == kActive && el[b].fine; },
-                 [=] __device__(int64_t b, int64_t, int64_t i) {
-                   const T v = mul_rn(static_cast<T>(el[b].g3), L[i]);
-                   L[i] = v >= T(3) ? v : T(3);
-                 });
-    }
-    // step 6: orientation and the element build
-    orientation_and_build();
-    // step 7: the ladders (S4), the weights
+    if (orient_out_) store_orientation();
+    // step 7: the ladders (S4); the weights, then steps 8-9: the sifts
     int32_t nrm = 0;
-    if (!ladder_and_weights(&nrm)) break;
-    // steps 8-9: the sifts
-    sifts(nrm);
+    if (!ladders(&nrm)) break;
+    sequence(2, nrm, [&] {
+      weights(nrm);
+      sifts(nrm);
+    });
     // step 10: the commit (S5); the next mode's L_prev is this L
     const bool more = commit();
     std::swap(L_, Lp_);
@@ -1670,6 +1747,14 @@ void run_chunk(const Geom& g, const Ctl& c, cudaStream_t s, Workspace& ws, const
                int32_t* hf, double* hp, double* he, std::vector<Elem>& out, T* orient) {
   Engine<T> e(g, c, s, ws);
   e.orient_out_ = g.dim >= 2 ? orient : nullptr;
+  // replayed launches: for calls that the launches bound (up to 1 M samples: 4 float64 images of
+  // 333 x 500 take 18.0 ms issued and 14.3 ms of kernels, 16 float32 ones of 512 x 512 37 and 36 ms);
+  // not for batches of uneven lengths (their lengths lie elsewhere on every call), nor while launches
+  // are counted
+  if (!g.len && g.batch * g.field <= (int64_t{1} << 20) && !profiling()) {
+    e.replays_ = ws.replays();
+    e.base_ = ws.base();
+  }
   const size_t lb = long_line_scratch_bytes(g, sizeof(T));
   const size_t rung_bytes = static_cast<size_t>(g.batch * g.field) * kMaxRungs * sizeof(T);
   if (long_totals_scratch_bytes(g, sizeof(T)) > rung_bytes) throw std::logic_error("edab: long-line totals exceed the rungs");
