@@ -11,16 +11,20 @@
 // cuFFT in float32, cpp/src/method/orientation.cu:674-767 of eda-cuda.) The basis is split once on
 // the host; the field tile is split in shared memory after its TMA load.
 //
-// Kernel (one 128 x 128 output tile per CTA, 192 threads):
+// Kernel (persistent: one CTA of 320 threads per SM runs 128 x 128 output tiles in turn):
 //   warp 4      TMA producer: A tile (128 rows x 32 floats, 128B swizzle) and the hi and lo basis
 //               tiles per k-block into a 3-stage ring (full / empty mbarriers);
 //   warps 0-3   split the A tile into hi and lo tiles (3xTF32: hi in place, 128B swizzle; BF16x3:
 //               two bfloat16 tiles of 64-byte rows in the 64B swizzle), fence the async proxy,
-//               arrive on the stage's split barrier; then the epilogue: tcgen05.ld of their TMEM
-//               lane quarter and the transposed store;
-//   warp 5      allocates 128 TMEM columns; one thread issues the split MMAs of every k-block
-//               (3 x 4 kind::tf32 with K = 8, or 3 x 2 kind::f16 with K = 16; M = N = 128) and
-//               commits each stage back to the producer.
+//               arrive on the stage's split barrier;
+//   warp 5      allocates 256 TMEM columns, two accumulators; one thread issues the split MMAs of
+//               every k-block (3 x 4 kind::tf32 with K = 8, or 3 x 2 kind::f16 with K = 16; M = N =
+//               128), commits each stage back to the producer and each tile to the epilogue;
+//   warps 6-9   the epilogue: tcgen05.ld of their TMEM lane quarter and the transposed store, while
+//               the next tile's products go to the other accumulator.
+// Bound by shared-memory bandwidth: the MMAs read 8 KB of operands each, and every k-block is written by
+// TMA, read and written by the split. 16 fields of 1000 x 768: 138 us per pass (154 us with one tile
+// per CTA, whose set-up, pipeline fill and epilogue stood in a row with its MMAs).
 // The store writes the tile transposed: the transformed axis becomes the slowest axis of the
 // element and the next axis the contiguous one (a rotation of the layout), so every transform of
 // the orientation reads K-major rows, and D passes bring a field back to its layout.
@@ -30,6 +34,7 @@
 
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -37,7 +42,7 @@ namespace edab {
 namespace tc {
 
 constexpr int kBM = 128, kBN = 128, kBK = 32, kStages = 3;
-constexpr int kThreadsTc = 192;
+constexpr int kThreadsTc = 320;
 constexpr unsigned long long kWaitNs = 2000000000ull;
 
 // The stage layout of a split mode. 3xTF32: [A hi (TMA, then split in place) | A lo | B hi | B lo],
@@ -178,7 +183,18 @@ struct RotOut {
   int64_t pitch_out;  // padded extent of the output's contiguous axis
   int64_t s_j;        // output stride of the transformed axis
   int64_t f_out;      // output samples per element
+  int32_t n_tiles;    // tiles along N
+  int64_t tiles;      // tiles of the pass
 };
+
+// Whether a tile of rows [m0, m0 + 128) holds a row of an element that runs.
+__device__ __forceinline__ bool tile_runs(const RotOut& ro, const int32_t* __restrict__ run, int64_t m0) {
+  const int64_t m1 = min(m0 + kBM, ro.M) - 1;
+  for (int64_t b = m0 / ro.rows; b <= m1 / ro.rows; ++b) {
+    if (run[b] != 0) return true;
+  }
+  return false;
+}
 
 template <bool BF16>
 __global__ void __launch_bounds__(kThreadsTc, 1)
@@ -188,33 +204,30 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + kStages * L::kBytes);
-  // bars: full[kStages], split[kStages], empty[kStages], acc
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 1);
-  __shared__ int32_t active_s;
+  // bars: full[kStages], split[kStages], empty[kStages], acc_full[2], acc_empty[2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 4);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t m0 = static_cast<int64_t>(blockIdx.y) * kBM;
-  const int32_t n0 = static_cast<int32_t>(blockIdx.x) * kBN;
+  const auto full_bar = [&](int i) { return smem_u32(&bars[i]); };
+  const auto split_bar = [&](int i) { return smem_u32(&bars[kStages + i]); };
+  const auto empty_bar = [&](int i) { return smem_u32(&bars[2 * kStages + i]); };
+  const auto acc_full = [&](int i) { return smem_u32(&bars[3 * kStages + i]); };
+  const auto acc_empty = [&](int i) { return smem_u32(&bars[3 * kStages + 2 + i]); };
   if (threadIdx.x == 0) {
-    // a tile whose rows all belong to elements that do not run is skipped
-    const int64_t m1 = min(m0 + kBM, ro.M) - 1;
-    int32_t act = 0;
-    for (int64_t b = m0 / ro.rows; b <= m1 / ro.rows; ++b) act |= run[b] != 0;
-    active_s = act;
-    if (act) {
-      for (int s = 0; s < kStages; ++s) {
-        mbar_init(smem_u32(&bars[s]), 1);
-        mbar_init(smem_u32(&bars[kStages + s]), 128);
-        mbar_init(smem_u32(&bars[2 * kStages + s]), 1);
-      }
-      mbar_init(smem_u32(&bars[3 * kStages]), 1);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(full_bar(i), 1);
+      mbar_init(split_bar(i), 128);
+      mbar_init(empty_bar(i), 1);
     }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(acc_full(i), 1);
+      mbar_init(acc_empty(i), 128);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  if (!active_s) return;
   if (warp == 5) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(kBN)
+                 "r"(2 * kBN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -222,122 +235,150 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  // Every role walks the CTA's tiles (those of elements that run) and counts k-blocks (it: the stage
+  // and phase of the ring) and tiles (j: the accumulator and its phase) alike.
   bool ok = true;
   if (warp == 4) {
     if (lane == 0) {
-      int32_t issued = 0;
-      for (int32_t kb = 0; kb < ro.kblocks; ++kb) {
-        const int s = kb % kStages;
-        const uint32_t ph = static_cast<uint32_t>(kb / kStages) & 1u;
-        if (!mbar_wait(smem_u32(&bars[2 * kStages + s]), ph ^ 1u)) {
-          ok = false;
-          break;
+      uint32_t it = 0;
+      for (int64_t t = blockIdx.x; ok && t < ro.tiles; t += gridDim.x) {
+        const int64_t m0 = t / ro.n_tiles * kBM;
+        const int32_t n0 = static_cast<int32_t>(t % ro.n_tiles) * kBN;
+        if (!tile_runs(ro, run, m0)) continue;
+        for (int32_t kb = 0; kb < ro.kblocks; ++kb, ++it) {
+          const int s = static_cast<int>(it % kStages);
+          if (!mbar_wait(empty_bar(s), ((it / kStages) & 1u) ^ 1u)) {
+            ok = false;
+            break;
+          }
+          unsigned char* st = base + s * L::kBytes;
+          mbar_expect_tx(full_bar(s), L::kTmaBytes);
+          tma_load_2d(smem_u32(st), &ta, kb * kBK, static_cast<int32_t>(m0), full_bar(s));
+          tma_load_2d(smem_u32(st + L::kBhi), &tb, kb * kBK, n0, full_bar(s));
+          tma_load_2d(smem_u32(st + L::kBlo), &tb, kb * kBK, ro.npad + n0, full_bar(s));
         }
-        unsigned char* st = base + s * L::kBytes;
-        const uint32_t full = smem_u32(&bars[s]);
-        mbar_expect_tx(full, L::kTmaBytes);
-        tma_load_2d(smem_u32(st), &ta, kb * kBK, static_cast<int32_t>(m0), full);
-        tma_load_2d(smem_u32(st + L::kBhi), &tb, kb * kBK, n0, full);
-        tma_load_2d(smem_u32(st + L::kBlo), &tb, kb * kBK, ro.npad + n0, full);
-        issued = kb + 1;
       }
       // the copies of the last stages complete before the CTA may leave
-      for (int32_t kb = max(0, issued - kStages); kb < issued; ++kb) {
-        if (!mbar_wait(smem_u32(&bars[kb % kStages]), static_cast<uint32_t>(kb / kStages) & 1u)) ok = false;
+      for (uint32_t k = it > kStages ? it - kStages : 0; k < it; ++k) {
+        if (!mbar_wait(full_bar(static_cast<int>(k % kStages)), (k / kStages) & 1u)) ok = false;
       }
     }
   } else if (warp == 5) {
     if (lane == 0) {
-      for (int32_t kb = 0; kb < ro.kblocks; ++kb) {
-        const int s = kb % kStages;
-        const uint32_t ph = static_cast<uint32_t>(kb / kStages) & 1u;
-        if (!mbar_wait(smem_u32(&bars[kStages + s]), ph)) {
+      uint32_t it = 0, j = 0;
+      for (int64_t t = blockIdx.x; ok && t < ro.tiles; t += gridDim.x) {
+        if (!tile_runs(ro, run, t / ro.n_tiles * kBM)) continue;
+        const int buf = static_cast<int>(j & 1u);
+        const uint32_t acc = tmem + static_cast<uint32_t>(buf * kBN);
+        if (!mbar_wait(acc_empty(buf), ((j >> 1) & 1u) ^ 1u)) {  // the epilogue has read it
           ok = false;
           break;
         }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t st = smem_u32(base + s * L::kBytes);
-        const uint32_t a_hi = st + L::kAhi, a_lo = st + L::kAlo, b_hi = st + L::kBhi, b_lo = st + L::kBlo;
-        if constexpr (BF16) {
+        for (int32_t kb = 0; kb < ro.kblocks; ++kb, ++it) {
+          const int s = static_cast<int>(it % kStages);
+          if (!mbar_wait(split_bar(s), (it / kStages) & 1u)) {
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t st = smem_u32(base + s * L::kBytes);
+          const uint32_t a_hi = st + L::kAhi, a_lo = st + L::kAlo, b_hi = st + L::kBhi, b_lo = st + L::kBlo;
+          if constexpr (BF16) {
 #pragma unroll
-          for (int kk = 0; kk < kBK / 16; ++kk) {
-            const uint32_t off = kk * 32;  // 16 bfloat16 of K inside the 64-byte swizzled row
-            mma_bf16(tmem, sw64_desc(a_hi + off), sw64_desc(b_hi + off), (kb | kk) != 0);
-            mma_bf16(tmem, sw64_desc(a_hi + off), sw64_desc(b_lo + off), 1u);
-            mma_bf16(tmem, sw64_desc(a_lo + off), sw64_desc(b_hi + off), 1u);
+            for (int kk = 0; kk < kBK / 16; ++kk) {
+              const uint32_t off = kk * 32;  // 16 bfloat16 of K inside the 64-byte swizzled row
+              mma_bf16(acc, sw64_desc(a_hi + off), sw64_desc(b_hi + off), (kb | kk) != 0);
+              mma_bf16(acc, sw64_desc(a_hi + off), sw64_desc(b_lo + off), 1u);
+              mma_bf16(acc, sw64_desc(a_lo + off), sw64_desc(b_hi + off), 1u);
+            }
+          } else {
+#pragma unroll
+            for (int kk = 0; kk < kBK / 8; ++kk) {
+              const uint32_t off = kk * 32;  // 8 tf32 of K inside the 128-byte swizzled row
+              mma_tf32(acc, sw128_desc(a_hi + off), sw128_desc(b_hi + off), (kb | kk) != 0);
+              mma_tf32(acc, sw128_desc(a_hi + off), sw128_desc(b_lo + off), 1u);
+              mma_tf32(acc, sw128_desc(a_lo + off), sw128_desc(b_hi + off), 1u);
+            }
+          }
+          mma_commit(empty_bar(s));
+        }
+        mma_commit(acc_full(buf));
+        ++j;
+      }
+    }
+  } else if (warp < 4) {
+    // warps 0-3: split the A tile of every stage
+    const int tid = threadIdx.x;  // 0..127
+    uint32_t it = 0;
+    for (int64_t t = blockIdx.x; ok && t < ro.tiles; t += gridDim.x) {
+      if (!tile_runs(ro, run, t / ro.n_tiles * kBM)) continue;
+      for (int32_t kb = 0; kb < ro.kblocks; ++kb, ++it) {
+        const int s = static_cast<int>(it % kStages);
+        if (!mbar_wait(full_bar(s), (it / kStages) & 1u)) {
+          ok = false;
+          break;
+        }
+        unsigned char* st = base + s * L::kBytes;
+        float4* a = reinterpret_cast<float4*>(st);
+        if constexpr (BF16) {
+          // the float32 tile (128-byte rows, 16-byte unit u of row r at unit u ^ (r & 7)) into the hi
+          // and lo bfloat16 tiles (64-byte rows, 16-byte unit u of row r at unit u ^ ((r >> 1) & 3))
+#pragma unroll
+          for (int i = 0; i < L::kTileF32 / 16 / 128; ++i) {
+            const int idx = tid + 128 * i;  // the physical float4 of the float32 tile
+            const int r = idx >> 3;
+            const int k0 = ((idx & 7) ^ (r & 7)) * 4;  // its first K column
+            const float4 v = a[idx];
+            const float f[4] = {v.x, v.y, v.z, v.w};
+            uint32_t hb[4], lb[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              hb[q] = bf16_bits(f[q]);
+              lb[q] = bf16_bits(__fsub_rn(f[q], bf16_value(hb[q])));
+            }
+            const int at = r * 64 + ((((k0 >> 3) ^ ((r >> 1) & 3))) << 4) + ((k0 & 7) << 1);
+            *reinterpret_cast<uint2*>(st + L::kAhi + at) = make_uint2(hb[0] | (hb[1] << 16), hb[2] | (hb[3] << 16));
+            *reinterpret_cast<uint2*>(st + L::kAlo + at) = make_uint2(lb[0] | (lb[1] << 16), lb[2] | (lb[3] << 16));
           }
         } else {
+          float4* alo = reinterpret_cast<float4*>(st + L::kAlo);
 #pragma unroll
-          for (int kk = 0; kk < kBK / 8; ++kk) {
-            const uint32_t off = kk * 32;  // 8 tf32 of K inside the 128-byte swizzled row
-            mma_tf32(tmem, sw128_desc(a_hi + off), sw128_desc(b_hi + off), (kb | kk) != 0);
-            mma_tf32(tmem, sw128_desc(a_hi + off), sw128_desc(b_lo + off), 1u);
-            mma_tf32(tmem, sw128_desc(a_lo + off), sw128_desc(b_hi + off), 1u);
+          for (int i = 0; i < L::kTileF32 / 16 / 128; ++i) {
+            const int idx = tid + 128 * i;
+            const float4 v = a[idx];
+            float4 h, l;
+            h.x = to_tf32(v.x);
+            h.y = to_tf32(v.y);
+            h.z = to_tf32(v.z);
+            h.w = to_tf32(v.w);
+            l.x = to_tf32(__fsub_rn(v.x, h.x));
+            l.y = to_tf32(__fsub_rn(v.y, h.y));
+            l.z = to_tf32(__fsub_rn(v.z, h.z));
+            l.w = to_tf32(__fsub_rn(v.w, h.w));
+            a[idx] = h;
+            alo[idx] = l;
           }
         }
-        mma_commit(smem_u32(&bars[2 * kStages + s]));
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_arrive(split_bar(s));
       }
-      mma_commit(smem_u32(&bars[3 * kStages]));
     }
   } else {
-    // warps 0-3: split the A tile of every stage, then the epilogue
-    const int t = threadIdx.x;  // 0..127
-    for (int32_t kb = 0; kb < ro.kblocks; ++kb) {
-      const int s = kb % kStages;
-      const uint32_t ph = static_cast<uint32_t>(kb / kStages) & 1u;
-      if (!mbar_wait(smem_u32(&bars[s]), ph)) {
+    // warps 6-9: the epilogue of every tile (warp w reads the TMEM lanes of quarter w mod 4)
+    const int quarter = warp & 3;
+    uint32_t j = 0;
+    for (int64_t t = blockIdx.x; ok && t < ro.tiles; t += gridDim.x) {
+      const int64_t m0 = t / ro.n_tiles * kBM;
+      const int32_t n0 = static_cast<int32_t>(t % ro.n_tiles) * kBN;
+      if (!tile_runs(ro, run, m0)) continue;
+      const int buf = static_cast<int>(j & 1u);
+      // the tcgen05.ld below is warp-collective: the warp decides together
+      if (!__all_sync(0xffffffffu, mbar_wait(acc_full(buf), (j >> 1) & 1u))) {
         ok = false;
         break;
       }
-      unsigned char* st = base + s * L::kBytes;
-      float4* a = reinterpret_cast<float4*>(st);
-      if constexpr (BF16) {
-        // the float32 tile (128-byte rows, 16-byte unit u of row r at unit u ^ (r & 7)) into the hi
-        // and lo bfloat16 tiles (64-byte rows, 16-byte unit u of row r at unit u ^ ((r >> 1) & 3))
-#pragma unroll
-        for (int i = 0; i < L::kTileF32 / 16 / 128; ++i) {
-          const int idx = t + 128 * i;  // the physical float4 of the float32 tile
-          const int r = idx >> 3;
-          const int k0 = ((idx & 7) ^ (r & 7)) * 4;  // its first K column
-          const float4 v = a[idx];
-          const float f[4] = {v.x, v.y, v.z, v.w};
-          uint32_t hb[4], lb[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            hb[q] = bf16_bits(f[q]);
-            lb[q] = bf16_bits(__fsub_rn(f[q], bf16_value(hb[q])));
-          }
-          const int at = r * 64 + ((((k0 >> 3) ^ ((r >> 1) & 3))) << 4) + ((k0 & 7) << 1);
-          *reinterpret_cast<uint2*>(st + L::kAhi + at) = make_uint2(hb[0] | (hb[1] << 16), hb[2] | (hb[3] << 16));
-          *reinterpret_cast<uint2*>(st + L::kAlo + at) = make_uint2(lb[0] | (lb[1] << 16), lb[2] | (lb[3] << 16));
-        }
-      } else {
-        float4* alo = reinterpret_cast<float4*>(st + L::kAlo);
-#pragma unroll
-        for (int i = 0; i < L::kTileF32 / 16 / 128; ++i) {
-          const int idx = t + 128 * i;
-          const float4 v = a[idx];
-          float4 h, l;
-          h.x = to_tf32(v.x);
-          h.y = to_tf32(v.y);
-          h.z = to_tf32(v.z);
-          h.w = to_tf32(v.w);
-          l.x = to_tf32(__fsub_rn(v.x, h.x));
-          l.y = to_tf32(__fsub_rn(v.y, h.y));
-          l.z = to_tf32(__fsub_rn(v.z, h.z));
-          l.w = to_tf32(__fsub_rn(v.w, h.w));
-          a[idx] = h;
-          alo[idx] = l;
-        }
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_arrive(smem_u32(&bars[kStages + s]));
-    }
-    // the tcgen05.ld below is warp-collective: the warp decides together
-    const bool acc_ready = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&bars[3 * kStages]), 0));
-    if (acc_ready) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int64_t m = m0 + warp * 32 + lane;
+      const int64_t m = m0 + quarter * 32 + lane;
       bool valid = m < ro.M;
       int64_t obase = 0;
       if (valid) {
@@ -349,17 +390,18 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
 #pragma unroll 1
       for (int c = 0; c < kBN / 32; ++c) {
         float v[32];
-        tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c * 32), v);
+        tmem_ld32(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * kBN + c * 32), v);
         if (valid) {
 #pragma unroll
           for (int jj = 0; jj < 32; ++jj) {
-            const int32_t j = n0 + c * 32 + jj;
-            if (j < ro.N) out[obase + static_cast<int64_t>(j) * ro.s_j] = v[jj];
+            const int32_t col = n0 + c * 32 + jj;
+            if (col < ro.N) out[obase + static_cast<int64_t>(col) * ro.s_j] = v[jj];
           }
         }
       }
-    } else {
-      ok = false;
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      mbar_arrive(acc_empty(buf));
+      ++j;
     }
   }
   if (!ok) atomicExch(err, 1);
@@ -367,7 +409,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
   __syncthreads();
   if (warp == 5) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kBN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kBN) : "memory");
   }
 }
 
@@ -439,9 +481,12 @@ void rot_pass_tc(cudaStream_t s, const RotPass& p, const void* basis, bool bf16,
   ro.pitch_out = p.pitch_out;
   ro.s_j = p.s_j;
   ro.f_out = p.f_out;
-  const int64_t mt = (p.M + tc::kBM - 1) / tc::kBM;
-  if (mt > 0x7fffffffLL) throw std::invalid_argument("eda: orientation pass too large");
-  const dim3 grid(static_cast<unsigned>((p.K + tc::kBN - 1) / tc::kBN), static_cast<unsigned>(mt));
+  ro.n_tiles = (p.K + tc::kBN - 1) / tc::kBN;
+  ro.tiles = (p.M + tc::kBM - 1) / tc::kBM * ro.n_tiles;
+  int sms = 148, dev = 0;
+  EDAB_CUDA(cudaGetDevice(&dev));
+  EDAB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const dim3 grid(static_cast<unsigned>(std::min<int64_t>(ro.tiles, sms)));
   if (bf16) {
     tc::set_smem_once<true>();
     tc::gemm_tc<true><<<grid, tc::kThreadsTc, tc::Stage<true>::kSmem, s>>>(ta, tb, ro, out, run, err);
