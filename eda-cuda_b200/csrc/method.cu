@@ -217,6 +217,49 @@ __device__ __forceinline__ double tie_tol(double tau, double amax) {
   return static_cast<double>(mul_rn(static_cast<T>(tau), static_cast<T>(amax)));
 }
 
+// The rung that G2's machine tests next (0: none).
+__device__ __forceinline__ int32_t g2_begin(const Elem& e) {
+  return (e.status == kActive && e.on_g2 && !e.g2_done) ? e.g2_rungs[e.g2_i] : 0;
+}
+// The outcome of a rung test (population p of np samples, the core and jump flags) and the machine's
+// next state (cpp/src/method/driver.cpp:73-116).
+__device__ __forceinline__ void g2_end(Elem& e, const Ctl& c, double p, int64_t np, int64_t count) {
+  e.g2_res_np = np;
+  e.g2_res_p = p;
+  e.g2_res_cov = __ddiv_rn(static_cast<double>(np), static_cast<double>(count));
+  if (np == 0 || !e.g2_any_core) e.g2_res_outcome = kG2None;
+  else if (__dmul_rn(c.fine_jump, p) > static_cast<double>(e.w)) e.g2_res_outcome = kG2Stop;
+  else e.g2_res_outcome = e.g2_any_jump ? kG2Accepted : kG2None;
+  const int32_t o = e.g2_res_outcome;
+  if (e.g2_pending) {
+    if (o == kG2Accepted) {
+      e.g2_done = 1;
+      e.g2_accepted = 1;
+      e.g2_acc_index = e.g2_i - 1;
+      return;
+    }
+    if (o == kG2Stop) {
+      e.g2_done = 1;
+      return;
+    }
+    e.g2_pending = 0;
+    ++e.g2_i;
+  } else {
+    if (o == kG2Stop) {
+      e.g2_done = 1;
+      return;
+    }
+    if (o == kG2Accepted) {
+      e.g2_pending = 1;
+      e.g2_cand_p = e.g2_res_p;
+      e.g2_cand_cov = e.g2_res_cov;
+      e.g2_cand_s = e.g2_rungs[e.g2_i];
+    }
+    ++e.g2_i;
+  }
+  if (e.g2_i >= e.g2_n && !e.g2_pending) e.g2_done = 1;
+}
+
 // d, e of a voxel (cpp/src/method/element.cuh:238-254): the cube side shrinks with the coherence c
 // and the segment half length takes up what the side gave away.
 template <class T>
@@ -890,7 +933,8 @@ void Engine<T>::local_floor() {
   });
 }
 
-// One G2 rung test of every element with srung > 0 (cpp/src/method/stats_rungs.cu:14-87).
+// One G2 rung test of every element with srung > 0 (cpp/src/method/stats_rungs.cu:14-87): the population
+// p (dsc_ + 4 B) and its count (cnt_), the flags of a core and of a jump. g2_begin set the windows.
 template <class T>
 void Engine<T>::g2_test(const uint8_t* ff, uint8_t* P) {
   const Ctl c = c_;
@@ -899,21 +943,6 @@ void Engine<T>::g2_test(const uint8_t* ff, uint8_t* P) {
   int32_t* wb = win(kG2b);
   int32_t* wcore = win(kG2core);
   int32_t* wrq = win(kG2rq);
-  for_elements(s_, B_, [=] __device__(int64_t b) {
-    const int32_t s = srung[b];
-    int32_t x = 0, y = 0, z = 0;
-    if (s > 0) {
-      const double sd = static_cast<double>(s);
-      x = odd_window(__dmul_rn(c.fine_beta, sd));
-      y = odd_window(__dmul_rn(c.fine_core, sd));
-      z = odd_window(__dmul_rn(__dmul_rn(2.0, c.absent_reach), static_cast<double>(x)));
-    }
-    wb[b] = x;
-    wcore[b] = y;
-    wrq[b] = z;
-    el[b].g2_any_core = 0;
-    el[b].g2_any_jump = 0;
-  });
   T* om = om2_;
   T* t1 = tmp1_;
   raw_window(ff, wb, srung, om, t1);
@@ -940,20 +969,8 @@ void Engine<T>::g2_test(const uint8_t* ff, uint8_t* P) {
   for_voxels(s_, g_, runS, [=] __device__(int64_t b, int64_t, int64_t i) {
     if (static_cast<double>(om[i]) > __dmul_rn(c.reset, p[b]) && t1[i] > T(0.5)) el[b].g2_any_jump = 1;
   });
-  const Geom g = g_;
-  for_elements(s_, B_, [=] __device__(int64_t b) {
-    if (srung[b] <= 0) return;
-    Elem& e = el[b];
-    e.g2_res_np = np[b];
-    e.g2_res_p = p[b];
-    e.g2_res_cov = __ddiv_rn(static_cast<double>(np[b]), static_cast<double>(elem_count(g, b)));
-    if (np[b] == 0 || !e.g2_any_core) e.g2_res_outcome = kG2None;
-    else if (__dmul_rn(c.fine_jump, p[b]) > static_cast<double>(e.w)) e.g2_res_outcome = kG2Stop;
-    else e.g2_res_outcome = e.g2_any_jump ? kG2Accepted : kG2None;
-  });
 }
 
-// G2 and G3 (cpp/src/method/driver.cpp:445-509; the machine of driver.cpp:73-116 on the device).
 // S1: the candidates of every G2-eligible element (host pow). Returns the rung tests to run (0: no element
 // has a candidate) and whether any element is active.
 template <class T>
@@ -997,44 +1014,35 @@ void Engine<T>::g2(int32_t steps) {
     ff = ff_;
   }
   int32_t* srung = mask(kSrung);
-  for (int32_t step = 0; step < steps; ++step) {
+  // The machine's steps: begin (the next rung's windows) and end (a test's outcome) of one test and the
+  // next share a launch.
+  const Ctl cc = c_;
+  const Geom gg = g_;
+  int32_t* wb = win(kG2b);
+  int32_t* wcore = win(kG2core);
+  int32_t* wrq = win(kG2rq);
+  const double* p = dsc_ + 4 * B_;
+  const int64_t* np = cnt_;
+  for (int32_t step = 0; step <= steps; ++step) {
+    const bool ends = step > 0;
     for_elements(s_, B_, [=] __device__(int64_t b) {
-      const Elem& e = el[b];
-      srung[b] = (e.status == kActive && e.on_g2 && !e.g2_done) ? e.g2_rungs[e.g2_i] : 0;
-    });
-    g2_test(ff, P_[step & 1]);
-    for_elements(s_, B_, [=] __device__(int64_t b) {
-      if (srung[b] <= 0) return;
-      Elem& e = el[b];
-      const int32_t o = e.g2_res_outcome;
-      if (e.g2_pending) {
-        if (o == kG2Accepted) {
-          e.g2_done = 1;
-          e.g2_accepted = 1;
-          e.g2_acc_index = e.g2_i - 1;
-          return;
-        }
-        if (o == kG2Stop) {
-          e.g2_done = 1;
-          return;
-        }
-        e.g2_pending = 0;
-        ++e.g2_i;
-      } else {
-        if (o == kG2Stop) {
-          e.g2_done = 1;
-          return;
-        }
-        if (o == kG2Accepted) {
-          e.g2_pending = 1;
-          e.g2_cand_p = e.g2_res_p;
-          e.g2_cand_cov = e.g2_res_cov;
-          e.g2_cand_s = e.g2_rungs[e.g2_i];
-        }
-        ++e.g2_i;
+      if (ends && srung[b] > 0) g2_end(el[b], cc, p[b], np[b], elem_count(gg, b));
+      const int32_t s = g2_begin(el[b]);
+      int32_t x = 0, y = 0, z = 0;
+      if (s > 0) {
+        const double sd = static_cast<double>(s);
+        x = odd_window(__dmul_rn(cc.fine_beta, sd));
+        y = odd_window(__dmul_rn(cc.fine_core, sd));
+        z = odd_window(__dmul_rn(__dmul_rn(2.0, cc.absent_reach), static_cast<double>(x)));
       }
-      if (e.g2_i >= e.g2_n && !e.g2_pending) e.g2_done = 1;
+      srung[b] = s;
+      wb[b] = x;
+      wcore[b] = y;
+      wrq[b] = z;
+      el[b].g2_any_core = 0;
+      el[b].g2_any_jump = 0;
     });
+    if (step < steps) g2_test(ff, P_[step & 1]);
   }
   // accepted: fine, p, the population of the accepted rung (step acc_index wrote P[acc_index & 1])
   int32_t* onfine = mask(kOnFine);

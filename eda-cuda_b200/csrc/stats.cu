@@ -555,16 +555,18 @@ __global__ void __launch_bounds__(TH) select_cluster(Geom g, SelView<T> a, const
 }
 
 // The grid-wide form for batches of few, large elements (select):
-// per digit, a counting launch over many CTAs per element (warp-aggregated shared-memory counts,
-// flushed with one global atomic per digit value and CTA) and a pick launch of one CTA per element
-// (the same block-wide prefix sum), the element's state in global memory between launches.
+// per digit, a launch over many CTAs per element (warp-aggregated shared-memory counts, flushed with
+// one global atomic per digit value and CTA) whose last CTA finds the digit by the same block-wide
+// prefix sum, the element's state in global memory between launches. (The pick was a launch of its
+// own: 6 and 12 launches per selection instead of 3 and 6, and two memsets instead of one.)
 template <class K>
 struct SelGridState {
   K prefix[2];
   unsigned long long rank[2];
   long long count;
   double gamma;
-  int32_t live, same;
+  int16_t live, same;
+  int32_t done;  // CTAs of the digit's launch that have added their counts
 };
 
 template <int KeyBits>
@@ -574,12 +576,85 @@ __device__ __forceinline__ void digit_of_pass(int pass, int* hi, int* shift, int
   *width = *hi - *shift;
 }
 
+// The digit of element b's ranks from its complete table tb (left zeroed), by one CTA.
+template <class K>
+__device__ __forceinline__ void grid_pick(int64_t b, SelGridState<K>* st, unsigned long long* tb, int32_t pass, double q,
+                                          double* out, int64_t* count_out) {
+  constexpr int kKeyBits = 8 * static_cast<int>(sizeof(K));
+  constexpr int kDigits = (kKeyBits + kDigitBits - 1) / kDigitBits;
+  __shared__ SelGridState<K> S;
+  __shared__ unsigned long long warp_tot[kThreads / 32];
+  __shared__ int hit_bin;
+  __shared__ unsigned long long hit_rest;
+  const int tid = threadIdx.x;
+  int hi, shift, width;
+  digit_of_pass<kKeyBits>(pass, &hi, &shift, &width);
+  const int bins = 1 << width;
+  if (pass == 0) {
+    unsigned long long n = 0;
+    for (int i = tid; i < bins; i += kThreads) n += tb[i];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) n += __shfl_xor_sync(0xffffffffu, n, d);
+    if ((tid & 31) == 0) warp_tot[tid >> 5] = n;
+    __syncthreads();
+    if (tid == 0) {
+      unsigned long long total = 0;
+      for (int w = 0; w < kThreads / 32; ++w) total += warp_tot[w];
+      S.prefix[0] = S.prefix[1] = K(0);
+      S.same = 1;
+      S.count = static_cast<long long>(total);
+      S.live = total > 0;
+      S.gamma = 0.0;
+      if (q < 0) {
+        S.rank[0] = total ? (total - 1) / 2 : 0;
+        S.rank[1] = total / 2;
+      } else if (total) {
+        long long i = 0, j = 0;
+        linear_index(static_cast<long long>(total), q, &i, &j, &S.gamma);
+        S.rank[0] = static_cast<unsigned long long>(i);
+        S.rank[1] = static_cast<unsigned long long>(j);
+      }
+    }
+  } else if (tid == 0) {
+    S = st[b];
+  }
+  __syncthreads();
+  const bool two = pass > 0 && !S.same;
+  if (S.live) {
+    for (int r = 0; r < 2; ++r) {
+      rank_digit<kThreads>(tb + (two ? r : 0) * kDigitBins, bins, S.rank[r], warp_tot, &hit_bin, &hit_rest);
+      if (tid == 0) {
+        S.prefix[r] |= static_cast<K>(hit_bin) << shift;
+        S.rank[r] = hit_rest;
+      }
+      __syncthreads();
+    }
+  }
+  for (int i = tid; i < 2 * kDigitBins; i += kThreads) tb[i] = 0ULL;  // clean for the next digit
+  if (tid == 0) {
+    S.same = S.prefix[0] == S.prefix[1];
+    S.done = 0;
+    st[b] = S;
+    if (!S.live) {  // no item: no later digit either
+      out[b] = d_nan();
+      if (count_out) count_out[b] = 0;
+    } else {
+      if (pass == kDigits - 1) {
+        const double v0 = key_value(S.prefix[0]), v1 = key_value(S.prefix[1]);
+        out[b] = q < 0 ? ((S.count & 1) ? v0 : __dmul_rn(__dadd_rn(v0, v1), 0.5)) : linear_between(v0, v1, S.gamma);
+        if (count_out) count_out[b] = S.count;
+      }
+    }
+  }
+}
+
 template <class T, class K>
 __global__ void __launch_bounds__(kThreads) select_grid_count(Geom g, SelView<T> a, const int32_t* run,
-                                                             const SelGridState<K>* st,
+                                                             SelGridState<K>* st,
                                                              unsigned long long* table, int32_t pass,
-                                                             SelCand<K> cand) {
+                                                             SelCand<K> cand, double q, double* out, int64_t* count_out) {
   __shared__ uint32_t local[2 * kDigitBins];
+  __shared__ int32_t last_s;
   const int64_t b = blockIdx.y;
   if (run && !run[b]) return;
   bool two = false;
@@ -629,80 +704,14 @@ __global__ void __launch_bounds__(kThreads) select_grid_count(Geom g, SelView<T>
     const uint32_t c = local[r * kDigitBins + (i - r * bins)];
     if (c) atomicAdd(&tb[r * kDigitBins + (i - r * bins)], static_cast<unsigned long long>(c));
   }
-}
-
-template <class K>
-__global__ void __launch_bounds__(kThreads) select_grid_pick(const int32_t* run, SelGridState<K>* st,
-                                                            unsigned long long* table, int32_t pass, double q,
-                                                            double* out, int64_t* count_out) {
-  constexpr int kKeyBits = 8 * static_cast<int>(sizeof(K));
-  constexpr int kDigits = (kKeyBits + kDigitBits - 1) / kDigitBits;
-  __shared__ SelGridState<K> S;
-  __shared__ unsigned long long warp_tot[kThreads / 32];
-  __shared__ int hit_bin;
-  __shared__ unsigned long long hit_rest;
-  const int64_t b = blockIdx.x;
-  if (run && !run[b]) return;
-  const int tid = threadIdx.x;
-  int hi, shift, width;
-  digit_of_pass<kKeyBits>(pass, &hi, &shift, &width);
-  const int bins = 1 << width;
-  unsigned long long* tb = table + static_cast<int64_t>(b) * 2 * kDigitBins;
-  if (pass == 0) {
-    unsigned long long n = 0;
-    for (int i = tid; i < bins; i += kThreads) n += tb[i];
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) n += __shfl_xor_sync(0xffffffffu, n, d);
-    if ((tid & 31) == 0) warp_tot[tid >> 5] = n;
-    __syncthreads();
-    if (tid == 0) {
-      unsigned long long total = 0;
-      for (int w = 0; w < kThreads / 32; ++w) total += warp_tot[w];
-      S.prefix[0] = S.prefix[1] = K(0);
-      S.same = 1;
-      S.count = static_cast<long long>(total);
-      S.live = total > 0;
-      S.gamma = 0.0;
-      if (q < 0) {
-        S.rank[0] = total ? (total - 1) / 2 : 0;
-        S.rank[1] = total / 2;
-      } else if (total) {
-        long long i = 0, j = 0;
-        linear_index(static_cast<long long>(total), q, &i, &j, &S.gamma);
-        S.rank[0] = static_cast<unsigned long long>(i);
-        S.rank[1] = static_cast<unsigned long long>(j);
-      }
-    }
-  } else if (tid == 0) {
-    S = st[b];
-  }
+  // the element's last CTA to get here has the whole table: it picks the digit
+  __threadfence();
   __syncthreads();
-  const bool two = pass > 0 && !S.same;
-  if (S.live) {
-    for (int r = 0; r < 2; ++r) {
-      rank_digit<kThreads>(tb + (two ? r : 0) * kDigitBins, bins, S.rank[r], warp_tot, &hit_bin, &hit_rest);
-      if (tid == 0) {
-        S.prefix[r] |= static_cast<K>(hit_bin) << shift;
-        S.rank[r] = hit_rest;
-      }
-      __syncthreads();
-    }
-  }
-  for (int i = tid; i < 2 * kDigitBins; i += kThreads) tb[i] = 0ULL;  // clean for the next digit
-  if (tid == 0) {
-    S.same = S.prefix[0] == S.prefix[1];
-    st[b] = S;
-    if (pass == kDigits - 1) {
-      if (!S.live) {
-        out[b] = d_nan();
-        if (count_out) count_out[b] = 0;
-      } else {
-        const double v0 = key_value(S.prefix[0]), v1 = key_value(S.prefix[1]);
-        out[b] = q < 0 ? ((S.count & 1) ? v0 : __dmul_rn(__dadd_rn(v0, v1), 0.5)) : linear_between(v0, v1, S.gamma);
-        if (count_out) count_out[b] = S.count;
-      }
-    }
-  }
+  if (tid == 0) last_s = atomicAdd(&st[b].done, 1) == static_cast<int32_t>(gridDim.x) - 1;
+  __syncthreads();
+  if (!last_s) return;
+  __threadfence();
+  grid_pick<K>(b, st, tb, pass, q, out, count_out);
 }
 
 // The split form for many items (select): one pass over the items instead of one per digit. A sample of
@@ -1014,8 +1023,8 @@ int32_t* split_mask(const Geom& g, const SelCand<K>& c) {
   return reinterpret_cast<int32_t*>(c.keys + static_cast<size_t>(g.batch) * c.cap);
 }
 
-// The grid-wide form: every digit a counting and a pick launch (scratch: the states, then the
-// [B][2][bins] count tables, zeroed here and left zeroed by every pick).
+// The grid-wide form: a launch per digit (scratch: the states, then the [B][2][bins] count tables,
+// zeroed here and left zeroed by every pick).
 template <class T, class K>
 void select_grid(cudaStream_t s, const Geom& g, const SelView<T>& a, double q, const int32_t* run, double* out,
                  int64_t* count, void* scratch, int sms) {
@@ -1023,21 +1032,21 @@ void select_grid(cudaStream_t s, const Geom& g, const SelView<T>& a, double q, c
   auto* st = static_cast<SelGridState<K>*>(scratch);
   auto* table = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) +
                                                        align256(static_cast<size_t>(g.batch) * sizeof(SelGridState<uint64_t>)));
-  EDAB_CUDA(cudaMemsetAsync(table, 0, static_cast<size_t>(g.batch) * 2 * kDigitBins * sizeof(unsigned long long), s));
+  // the states, the tables and the candidates' counts lie one after the other
+  const SelCand<K> cand = (sizeof(K) == 8 || EDAB_SEL_CAND32) ? cand_of<K>(g, scratch) : SelCand<K>{};
+  const size_t clear = static_cast<size_t>(reinterpret_cast<char*>(cand_of<K>(g, scratch).n) - static_cast<char*>(scratch)) +
+                       static_cast<size_t>(g.batch) * sizeof(unsigned long long);
+  EDAB_CUDA(cudaMemsetAsync(scratch, 0, clear, s));
   // CTAs per element: 64 items per thread, and for small batches enough CTAs for 8 per SM (at
   // least 4 items per thread)
   const int64_t by_items = (a.items + int64_t{kThreads} * 64 - 1) / (int64_t{kThreads} * 64);
   const int64_t fill = std::min<int64_t>((int64_t{8} * sms + g.batch - 1) / g.batch,
                                          std::max<int64_t>(1, a.items / (int64_t{kThreads} * 4)));
   const unsigned ctas = static_cast<unsigned>(std::clamp<int64_t>(std::max(by_items, fill), 1, 1024));
-  const SelCand<K> cand = (sizeof(K) == 8 || EDAB_SEL_CAND32) ? cand_of<K>(g, scratch) : SelCand<K>{};
-  if (cand.keys) EDAB_CUDA(cudaMemsetAsync(cand.n, 0, static_cast<size_t>(g.batch) * sizeof(unsigned long long), s));
   for (int pass = 0; pass < kDigits; ++pass) {
     select_grid_count<T, K><<<dim3(ctas, static_cast<unsigned>(g.batch)), kThreads, 0, s>>>(g, a, run, st, table, pass,
-                                                                                          cand);
+                                                                                          cand, q, out, count);
     EDAB_LAUNCH("select_grid_count");
-    select_grid_pick<K><<<static_cast<unsigned>(g.batch), kThreads, 0, s>>>(run, st, table, pass, q, out, count);
-    EDAB_LAUNCH("select_grid_pick");
   }
 }
 
@@ -1079,8 +1088,8 @@ void select(cudaStream_t s, const Geom& g, const Sel<T>& sel, double q, const in
   // Clusters (one launch): of 256-thread CTAs when the batch fills the GPU with them, else of
   // 1024-thread CTAs while an element has at most 8 items for each of their threads (a median of 2048
   // samples: 13 us and one launch, against 8 launches of 3 us); larger elements of small batches take
-  // the grid-wide form, two launches per digit over many CTAs (133 000 items: 40 us, against 54 us in
-  // one cluster).
+  // the grid-wide form, a launch per digit over many CTAs (133 000 items: 40 us, against 54 us in one
+  // cluster).
   int sms = 148;
   {
     int dev = 0;
