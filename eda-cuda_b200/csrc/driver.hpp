@@ -68,16 +68,8 @@ class HostStaging {
   ~HostStaging();
   unsigned char* piece(int i);  // i = 0 or 1
   void release();
-  // The launch sequences replayed on this buffer, for a workspace that lives as long as its thread
-  // (nullptr: a view of the caller's memory, or a workspace that ragged batches' workers lease, which
-  // meets other shapes on every call).
-  Replays* replays() { return keeps_replays_ ? &replays_ : nullptr; }
-  void keep_replays() { keeps_replays_ = true; }
-  const void* base() const { return base_; }
 
  private:
-  Replays replays_;
-  bool keeps_replays_ = false;
   unsigned char* base_ = nullptr;
 };
 HostStaging& thread_staging();

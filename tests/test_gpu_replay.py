@@ -1,0 +1,109 @@
+# SPDX-License-Identifier: Apache-2.0
+"""Replayed launch sequences (replay.hpp) give what the same launches issued one by one give, bit for
+bit: the first, second and later calls of a geometry, on other data each time; geometries in turn,
+more of them than the cache keeps; another constant of the call; fields that fail; other streams and
+threads; both sides of the size rule. Calls whose launches are counted (eda_profile) issue every one."""
+
+from __future__ import annotations
+
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from eda import _native
+
+    return ctypes.CDLL(str(_native.LIB))
+
+
+def field(shape, dtype, seed):
+    rng = np.random.default_rng(seed)
+    x = rng.standard_normal(shape)
+    for a in range(1, len(shape)):
+        t = np.arange(shape[a]).reshape([-1 if k == a else 1 for k in range(len(shape))])
+        x = x + np.sin(2 * np.pi * t / rng.uniform(9, 30)) + 2 * np.sin(2 * np.pi * t / rng.uniform(50, 90))
+    return x.astype(dtype)
+
+
+def results(x, **kw):
+    import eda
+
+    y, info = eda.decompose(x, axes=tuple(range(1, x.ndim)), return_info=True, errors="status", **kw)
+    y = y.cpu().numpy() if hasattr(y, "cpu") else np.asarray(y)
+    return [y] + [np.asarray(getattr(info, k)) for k in ("n_imfs", "error", "windows", "sifts", "spacing", "energy")]
+
+
+def issued(lib, x, **kw):
+    lib.eda_profile(1)
+    try:
+        return results(x, **kw)
+    finally:
+        lib.eda_profile(0)
+
+
+def check(lib, x, **kw):
+    got, want = results(x, **kw), issued(lib, x, **kw)
+    for a, b in zip(got, want):
+        assert a.shape == b.shape and a.tobytes() == b.tobytes()
+
+
+SHAPES = [(1, 2048), (3, 300), (2, 41, 67), (3, 9, 14, 33), (1, 2), (70, 513), (1, 20011)]
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("shape", SHAPES, ids=["x".join(map(str, s)) for s in SHAPES])
+def test_calls_of_one_geometry(lib, shape, dtype):
+    for seed in range(4):
+        x = field(shape, dtype, seed)
+        if seed == 1:
+            x[-1] = 0.5  # a field without modes beside the others
+        if seed == 2:
+            x[0].reshape(-1)[1] = np.nan  # one that fails
+        check(lib, x)
+
+
+def test_geometries_and_constants_in_turn(lib):
+    for seed in range(2):
+        for shape in SHAPES:  # (each has several sequences: more than the cache keeps)
+            for kw in ({}, {"max_imf": 2}, {"tie_tolerance": 0.01}, {"check_finite": False}):
+                check(lib, field(shape, np.float32, seed), **kw)
+
+
+@pytest.mark.parametrize("shape", [(4, 512, 512), (5, 512, 512)], ids=["at the limit", "above"])
+def test_size_rule(lib, shape):
+    for seed in range(2):
+        check(lib, field(shape, np.float32, seed), max_imf=2)
+
+
+def test_streams_and_threads(lib):
+    import torch
+
+    xs = [field((2, 700), np.float32, s) for s in range(6)]
+    want = [issued(lib, x) for x in xs]
+    wrong = []
+
+    def work(k):
+        stream = torch.cuda.Stream()
+        for rep in range(3):
+            for i in range(len(xs)):
+                j = (i + k) % len(xs)
+                with torch.cuda.stream(stream if rep else torch.cuda.current_stream()):
+                    got = results(torch.from_numpy(xs[j]).cuda())
+                if any(a.tobytes() != b.tobytes() for a, b in zip(got, want[j])):
+                    wrong.append((k, rep, j))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
