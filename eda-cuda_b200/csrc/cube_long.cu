@@ -5,17 +5,20 @@
 // the staged passes (cube_ext.cu, cube_box.cu).
 //
 // Max / min: the scratch holds the extreme of every 32-sample block. A tile computes the block
-// suffixes H where its windows begin and the block prefixes G where they end (by warp shuffles),
-// doubles the block extremes to runs of 2^k blocks, two of which cover the blocks between, and takes
-// four reads per output whatever the window. Two launches.
+// suffixes H where its windows begin and the block prefixes G where they end (a lane per block, in shared
+// memory: three instructions per sample of 32 lanes; by warp shuffles they were twenty), doubles the
+// extremes of the blocks that its windows reach to runs of 2^k blocks, two of which cover the blocks
+// between, and takes four reads per output whatever the window. Two launches.
 // Box sums: a tile folds the 32-sample chunks where its windows begin (H, the reversed line) and end
 // (G). Short segments (at most a quarter tile) are folded from their start inside the tile; the
 // carries of longer ones come from a table of the line's chunk totals, summed per segment in chunk
-// order by the last CTA of the totals' launch. Three launches.
+// order by the last CTA of the totals' launch. Two launches, three where the samples have to be copied
+// (bit fields, outputs over the input).
 // What bounds them: at small batches the launches themselves, else the output loops' issue slots and
-// the folds' shared-memory round trips; the samples lie in L2 after the first launch. 16 lines of
-// 40 000 float32 samples, max and min: 18 us at windows of 15, 25 us at 9001 (23 and 147 us with whole
-// segments staged per tile and five launches for the widest windows); box sums 13 and 35 us (17, 82).
+// the folds' shared-memory round trips; the samples lie in L2 after the first launch. A batch of 1024
+// signals of 256 to 65 536 float32 samples: max and min 147 -> 89 us per launch, the copies 25.6 -> 15.2 ms
+// in all, box sums 88 -> 80 us (tiles of 2048 outputs: 76 us, but the totals 29 -> 37 us). Totals from
+// coalesced tiles instead of a lane per chunk: 31 us either way, float64 6.4 -> 9.2 us; not kept.
 #include "cube.cuh"
 
 #include <algorithm>
@@ -100,7 +103,26 @@ __global__ void __launch_bounds__(kThreads) long_input(Geom g, PassArgs<T> a, Lo
 // The block length of half width r: B <= 2r, at most 32.
 __device__ __forceinline__ int32_t long_block(int32_t r) { return r >= 16 ? 32 : 2 << (31 - __clz(max(r, 1))); }
 
-// dynamic shared memory: H, G [span], S0, S1, PB [nbp]; span = tile + 128
+// A staged sample's word: a lane's 32 samples lie one word further than its neighbour's.
+__host__ __device__ constexpr int32_t padded(int32_t i) { return i + (i >> 5); }
+// Words of the samples that a tile stages where its windows begin, or end.
+__host__ __device__ constexpr int32_t ext_words(int32_t tile) { return padded(tile + 128); }
+
+// The extremes of the 32 staged samples at x (32 words) from each to its block's end (DOWN) or from its
+// block's start on, in place.
+template <bool DOWN, class K>
+__device__ __forceinline__ void scan_blocks(K* x, int32_t B) {
+  K v = key_min<K>();
+#pragma unroll
+  for (int u = 0; u < 32; ++u) {
+    const int i = DOWN ? 31 - u : u;
+    if (B < 32 && (u & (B - 1)) == 0) v = key_min<K>();
+    v = max(v, x[i]);
+    x[i] = v;
+  }
+}
+
+// dynamic shared memory: H, G [ext_words], S0, S1, PB [nbp]
 template <class T>
 __global__ void __launch_bounds__(kThreads) long_ext(Geom g, PassArgs<T> a, LongScratch<T> L, int32_t tile) {
   using K = typename KeyType<T>::type;
@@ -128,7 +150,7 @@ __global__ void __launch_bounds__(kThreads) long_ext(Geom g, PassArgs<T> a, Long
     for (int32_t x = X0 + threadIdx.x; x < end; x += kThreads) out[x] = x < n ? key_back(line[x]) : T(0);
     return;
   }
-  const int32_t span = tile + 128, nbp = static_cast<int32_t>(g.pitch >> 5);
+  const int32_t span = ext_words(tile), nbp = static_cast<int32_t>(g.pitch >> 5);
   K* H = reinterpret_cast<K*>(smem_raw);
   K* G = H + span;
   K* S = G + span;
@@ -139,39 +161,27 @@ __global__ void __launch_bounds__(kThreads) long_ext(Geom g, PassArgs<T> a, Long
   // block between is read from H), G over the blocks of the windows' ends
   const int32_t h0 = max(X0 - r, 0) >> 5 << 5, h1 = min(n, ((max(X1 - 1 - r, 0) + 2 * B) >> 5) * 32 + 32);
   const int32_t g0 = min(X0 + r, n - 1) >> 5 << 5, g1 = min(n, (min(X1 - 1 + r, n - 1) >> 5) * 32 + 32);
-  for (int32_t i0 = h0 + 32 * warp; i0 < h1; i0 += kThreads) {
-    const int32_t i = i0 + lane;
-    K v = i < n ? line[i] ^ nm : idn;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      if (d < B) {
-        const K o = __shfl_down_sync(0xffffffffu, v, d);
-        if ((lane & (B - 1)) + d < B) v = max(v, o);
-      }
-    }
-    H[i - h0] = v;
+  for (int32_t i = h0 + threadIdx.x; i < h1; i += kThreads) H[padded(i - h0)] = line[i] ^ nm;
+  for (int32_t i = g0 + threadIdx.x; i < g1; i += kThreads) G[padded(i - g0)] = line[i] ^ nm;
+  const int32_t hb = (h1 - h0 + 31) >> 5, gb = (g1 - g0 + 31) >> 5;
+  for (int32_t i = h1 + threadIdx.x; i < h0 + 32 * hb; i += kThreads) H[padded(i - h0)] = idn;
+  for (int32_t i = g1 + threadIdx.x; i < g0 + 32 * gb; i += kThreads) G[padded(i - g0)] = idn;
+  // the blocks that the tile's windows reach, and their extremes (B == 32)
+  const int32_t bs = max(X0 - r, 0) >> 5, be = (min(X1 - 1 + r, n - 1) >> 5) + 1;
+  if (B == 32) {
+    const K* from = L.blocks + (is_min ? g.batch + b : b) * nbp;
+    for (int32_t i = bs + threadIdx.x; i < be; i += kThreads) S[i] = from[i];
   }
-  for (int32_t i0 = g0 + 32 * warp; i0 < g1; i0 += kThreads) {
-    const int32_t i = i0 + lane;
-    K v = i < n ? line[i] ^ nm : idn;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      if (d < B) {
-        const K o = __shfl_up_sync(0xffffffffu, v, d);
-        if ((lane & (B - 1)) >= d) v = max(v, o);
-      }
-    }
-    G[i - g0] = v;
+  __syncthreads();
+  for (int32_t t = threadIdx.x; t < hb + gb; t += kThreads) {
+    if (t < hb) scan_blocks<true>(H + 33 * t, B);
+    else scan_blocks<false>(G + 33 * (t - hb), B);
   }
   int32_t run = 0;  // B == 32: S holds the extremes of runs of 2^run blocks
   if (B == 32) {
-    const int32_t nb = (n + 31) >> 5;
-    const K* from = L.blocks + (is_min ? g.batch + b : b) * nbp;
-    for (int32_t i = threadIdx.x; i < nb; i += kThreads) S[i] = from[i];
-    __syncthreads();
     if (X0 < r) {  // some windows begin before the line: the extremes of the blocks up to each
-      const int32_t per = (nb + kThreads - 1) / kThreads;
-      const int32_t c0 = min(static_cast<int32_t>(threadIdx.x) * per, nb), c1 = min(c0 + per, nb);
+      const int32_t per = (be + kThreads - 1) / kThreads;
+      const int32_t c0 = min(static_cast<int32_t>(threadIdx.x) * per, be), c1 = min(c0 + per, be);
       K run_max = idn;
       for (int32_t i = c0; i < c1; ++i) run_max = max(run_max, S[i]);
       K scan = run_max;
@@ -193,7 +203,7 @@ __global__ void __launch_bounds__(kThreads) long_ext(Geom g, PassArgs<T> a, Long
     const int32_t least = (r >> 4) - 1;  // whole blocks that every window inside the line holds
     while ((2 << run) <= least) {
       const int32_t half = 1 << run;
-      for (int32_t i = threadIdx.x; i < nb; i += kThreads) S2[i] = max(S[i], S[min(i + half, nb - 1)]);
+      for (int32_t i = bs + threadIdx.x; i < be; i += kThreads) S2[i] = max(S[i], S[min(i + half, be - 1)]);
       __syncthreads();
       K* t = S;
       S = S2;
@@ -207,10 +217,10 @@ __global__ void __launch_bounds__(kThreads) long_ext(Geom g, PassArgs<T> a, Long
     if (x < n) {
       const int32_t lo = x - r, hi = min(x + r, n - 1);
       const int32_t b0 = lo >= 0 ? lo >> sh : -1, b1 = hi >> sh;
-      K y = lo >= 0 ? H[lo - h0] : idn;
-      if (b1 > b0) y = max(y, G[hi - g0]);
+      K y = lo >= 0 ? H[padded(lo - h0)] : idn;
+      if (b1 > b0) y = max(y, G[padded(hi - g0)]);
       if (b1 - b0 > 1) {
-        if (B < 32) y = max(y, H[((b0 + 1) << sh) - h0]);
+        if (B < 32) y = max(y, H[padded(((b0 + 1) << sh) - h0)]);
         else if (lo < 0) y = max(y, PB[b1 - 1]);
         else y = max(y, max(S[b0 + 1], S[max(b0 + 1, b1 - (1 << run))]));
       }
@@ -418,8 +428,15 @@ __global__ void __launch_bounds__(kThreads) long_box(Geom g, PassArgs<T> a, Long
   T* TH = TG + side_chunks(tile);
   // (within the bounds for every length, window and tile, checked on the CPU)
   if (max(sg.len, sh.len) > side_samples(tile) || max(sg.chunks, sh.chunks) > side_chunks(tile)) return;
-  for (int32_t i = threadIdx.x; i < sg.len; i += kThreads) RG[i + (i >> 5)] = line[reflect_index(sg.e0 + i, n)];
-  for (int32_t i = threadIdx.x; i < sh.len; i += kThreads) RH[i + (i >> 5)] = line[n - 1 - reflect_index(sh.e0 + i, n)];
+  if (min(sg.e0, sh.e0) >= 0 && max(sg.e0 + sg.len, sh.e0 + sh.len) <= n) {  // no sample is a reflected one
+    const T* from = line + sg.e0;
+    for (int32_t i = threadIdx.x; i < sg.len; i += kThreads) RG[padded(i)] = from[i];
+    from = line + (n - 1 - sh.e0);
+    for (int32_t i = threadIdx.x; i < sh.len; i += kThreads) RH[padded(i)] = from[-i];
+  } else {
+    for (int32_t i = threadIdx.x; i < sg.len; i += kThreads) RG[padded(i)] = line[reflect_index(sg.e0 + i, n)];
+    for (int32_t i = threadIdx.x; i < sh.len; i += kThreads) RH[padded(i)] = line[n - 1 - reflect_index(sh.e0 + i, n)];
+  }
   __syncthreads();
   const int32_t all = sg.chunks + sh.chunks;
   for (int32_t t = threadIdx.x; t < all; t += kThreads) {
@@ -512,12 +529,19 @@ void launch_long(cudaStream_t s, const Geom& g, const PassArgs<T>& a, void* line
   L.done = reinterpret_cast<int32_t*>(static_cast<char*>(totals) + static_cast<size_t>(kMaxRungs) * g.batch * 2 * L.TSL * sizeof(T));
   const unsigned B = static_cast<unsigned>(g.batch);
   const unsigned in_x = static_cast<unsigned>(std::clamp<int64_t>((g.pitch + 4 * kThreads - 1) / (4 * kThreads), 1, 64));
-  long_input<T><<<dim3(in_x, B), kThreads, 0, s>>>(g, a, L, box ? a.rungs * static_cast<int32_t>(g.batch) : 0);
-  EDAB_LAUNCH("long_input");
+  // box sums read their input where it lies, unless it is a bit field or an output overwrites it
+  const T* out_end = a.out0 + (a.rungs - 1) * a.out_stride + g.batch * g.field;
+  if (box && !a.bits && (a.in0 >= out_end || a.in0 + g.batch * g.field <= a.out0)) {
+    L.line = const_cast<T*>(a.in0);
+    EDAB_CUDA(cudaMemsetAsync(L.done, 0, static_cast<size_t>(a.rungs) * B * sizeof(int32_t), s));
+  } else {
+    long_input<T><<<dim3(in_x, B), kThreads, 0, s>>>(g, a, L, box ? a.rungs * static_cast<int32_t>(g.batch) : 0);
+    EDAB_LAUNCH("long_input");
+  }
   const int32_t tile = long_tile(g, static_cast<int64_t>(a.rungs) * nf, sms);
   const unsigned tiles = static_cast<unsigned>((g.n_last + tile - 1) / tile);
   if (!box) {
-    const size_t smem = (static_cast<size_t>(2) * (tile + 128) + 3 * static_cast<size_t>(g.pitch / 32)) * sizeof(T);
+    const size_t smem = (static_cast<size_t>(2) * ext_words(tile) + 3 * static_cast<size_t>(g.pitch / 32)) * sizeof(T);
     if (smem > smem_cap) throw std::invalid_argument("edab: a line is too long for the long-line cube pass");
     once_on_device(reinterpret_cast<const void*>(long_ext<T>), [&] {
       EDAB_CUDA(cudaFuncSetAttribute(long_ext<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_cap)));
