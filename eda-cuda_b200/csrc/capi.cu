@@ -154,6 +154,32 @@ int eda_ragged_element(const eda_ragged_run* run, int64_t i, int32_t* rows, int3
   });
 }
 
+int eda_ragged_elements(const eda_ragged_run* run, int32_t* rows, int32_t* n_imfs, int32_t* error, int32_t* windows,
+                        int32_t* sifts, double* spacing, double* energy) {
+  return guarded([&] {
+    if (!run) throw std::invalid_argument("eda: null run");
+    const edab::RaggedRun& R = *run->run;
+    size_t to = 0;
+    for (size_t i = 0; i < R.group.size(); ++i) {
+      const edab::Run& r = *R.groups[static_cast<size_t>(R.group[i])];
+      const int64_t j = R.index[i];
+      const size_t at = static_cast<size_t>(j) * static_cast<size_t>(r.rows_cap > 0 ? r.rows_cap - 1 : 0);
+      const int32_t err = r.error[static_cast<size_t>(j)];
+      const size_t k = err ? 0 : static_cast<size_t>(r.n_imfs[static_cast<size_t>(j)]);
+      if (rows) rows[i] = r.rows_of(j);
+      if (n_imfs) n_imfs[i] = r.n_imfs[static_cast<size_t>(j)];
+      if (error) error[i] = err;
+      for (size_t m = 0; m < k; ++m) {
+        if (windows) windows[to + m] = r.hist_scale[at + m];
+        if (sifts) sifts[to + m] = r.hist_sifts[at + m];
+        if (spacing) spacing[to + m] = r.hist_spacing[at + m];
+        if (energy) energy[to + m] = r.hist_energy[at + m];
+      }
+      to += k;
+    }
+  });
+}
+
 int eda_ragged_collect(eda_ragged_run* run, int64_t i, void* dst, int dst_on_device, void* stream) {
   return guarded([&] {
     if (!run || !dst) throw std::invalid_argument("eda: null argument");

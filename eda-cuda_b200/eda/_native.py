@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes
 import json
+import math
 from pathlib import Path
 from typing import Any
 
@@ -72,6 +73,7 @@ class Core:
         L.eda_decompose_ragged.argtypes = [ctypes.POINTER(vp), ctypes.c_int, ctypes.c_int, ctypes.c_int, i64,
                                            ctypes.POINTER(i64), ctypes.POINTER(_Params), i32, vp, ctypes.POINTER(vp)]
         L.eda_ragged_element.argtypes = [vp, i64] + [vp] * 7
+        L.eda_ragged_elements.argtypes = [vp] * 8
         L.eda_ragged_collect.argtypes = [vp, i64, vp, ctypes.c_int, vp]
         L.eda_ragged_collect_all.argtypes = [vp, vp, ctypes.c_int, ctypes.POINTER(i64), vp]
         L.eda_monogenic.argtypes = [vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, i64, ctypes.POINTER(i64), i64, vp,
@@ -323,23 +325,22 @@ class Core:
         code = 0 if np.dtype(dtype) == np.float32 else 1
         self._check(self._lib.eda_decompose_ragged(xs, int(on_device), code, dim, count, n, ctypes.byref(p),
                                                    int(workers), ctypes.c_void_p(stream), ctypes.byref(run)))
-        infos, rows_of = [], []
+        infos = []
         try:
-            for i in range(count):
-                P, k, err = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int32()
-                self._check(self._lib.eda_ragged_element(run, i, ctypes.byref(P), ctypes.byref(k), ctypes.byref(err),
-                                                         None, None, None, None))
-                K = 0 if err.value else k.value
-                info = {"n_imfs": int(k.value), "error": int(err.value), "windows": np.zeros(K, np.int32),
-                        "sifts": np.zeros(K, np.int32), "spacing": np.zeros(K, np.float64),
-                        "energy": np.zeros(K, np.float64)}
-                if K:
-                    self._check(self._lib.eda_ragged_element(
-                        run, i, None, None, None, *(ctypes.c_void_p(info[f].ctypes.data) for f in
-                                                    ("windows", "sifts", "spacing", "energy"))))
+            # every element's information in one native call (two per element took 9 ms for 1024 signals)
+            rows_of, n_imfs, error = (np.zeros(count, np.int32) for _ in range(3))
+            ints = [ctypes.c_void_p(a.ctypes.data) for a in (rows_of, n_imfs, error)]
+            self._check(self._lib.eda_ragged_elements(run, *ints, None, None, None, None))
+            ends = [0] + np.cumsum(np.where(error != 0, 0, n_imfs)).tolist()
+            per_imf = {f: np.zeros(ends[-1], t) for f, t in (("windows", np.int32), ("sifts", np.int32),
+                                                             ("spacing", np.float64), ("energy", np.float64))}
+            self._check(self._lib.eda_ragged_elements(run, None, None, None,
+                                                      *(ctypes.c_void_p(a.ctypes.data) for a in per_imf.values())))
+            for i, (k, err) in enumerate(zip(n_imfs.tolist(), error.tolist())):
+                info = {f: a[ends[i]:ends[i + 1]] for f, a in per_imf.items()}
+                info["n_imfs"], info["error"] = k, err
                 infos.append(info)
-                rows_of.append(int(P.value))
-            sizes = [P * int(np.prod(sh)) for P, sh in zip(rows_of, shapes)]
+            sizes = [P * math.prod(sh) for P, sh in zip(rows_of.tolist(), shapes)]
             offsets = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64) if count else np.zeros(1, np.int64)
             buf, ptr = alloc(int(offsets[-1]))
             if count:
@@ -348,9 +349,8 @@ class Core:
                     ctypes.c_void_p(stream)))
         finally:
             self._lib.eda_ragged_free(run)
-        return [(buf[int(offsets[i]):int(offsets[i + 1])].reshape((rows_of[i],) + tuple(shapes[i])), infos[i])
-                for i in range(count)]
-
+        at = offsets.tolist()
+        return [(buf[at[i]:at[i + 1]].reshape((P,) + tuple(shapes[i])), infos[i]) for i, P in enumerate(rows_of.tolist())]
 
     def monogenic(self, ptr: int, on_device: bool, dtype: str, shape: tuple[int, ...], stream: int, out_ptr: int,
                   max_chunk: int = 0) -> np.ndarray:

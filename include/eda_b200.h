@@ -157,6 +157,11 @@ EDA_API int eda_decompose_ragged(const void* const* x, int x_on_device, int dtyp
  * sifts, spacing, energy (n_imfs entries each, none for a failed element; any pointer may be NULL). */
 EDA_API int eda_ragged_element(const eda_ragged_run* run, int64_t i, int32_t* rows, int32_t* n_imfs, int32_t* error,
                                int32_t* windows, int32_t* sifts, double* spacing, double* energy);
+/* The same of every element, in one call: rows, n_imfs and error [count], and the windows, sifts,
+ * spacing and energy of all elements one after the other (n_imfs entries of each, none of a failed
+ * element; any pointer may be NULL). */
+EDA_API int eda_ragged_elements(const eda_ragged_run* run, int32_t* rows, int32_t* n_imfs, int32_t* error,
+                                int32_t* windows, int32_t* sifts, double* spacing, double* energy);
 /* Element i's rows (P, *n_i) into dst (host, or device memory of the run's device), complete on
  * return: a NaN row for a failed element, the IMFs then the residue otherwise. */
 EDA_API int eda_ragged_collect(eda_ragged_run* run, int64_t i, void* dst, int dst_on_device, void* stream);
