@@ -57,7 +57,7 @@ struct StepTree {
   }
 };
 
-// One step of a row: the warp's tree over the chunks [32 step, 32 step + 32), staged by coalesced loads
+// One step of a row: the warp's tree over the chunks [32 step, 32 step + 32), staged by coalesced 16-byte loads
 // and padded with zeros (+0 changes no sum of squares); the lane's max |v| (as T's bits) and whether a
 // sample is not finite are added to amax and bad (counted).
 template <class T>
@@ -70,10 +70,30 @@ __device__ __forceinline__ double row_step(const T* __restrict__ row, int32_t n,
   const int lane = threadIdx.x & 31;
   const int32_t i0 = step * 1024, left = min(n - i0, 1024);
   __syncwarp();
-#pragma unroll 8
-  for (int32_t c = 0; c < 32; ++c) {
-    const int32_t i = 32 * c + lane;
-    if (32 * c < left) tile[33 * c + lane] = i < left ? row[i0 + i] : T(0);
+  // 16 bytes per lane and load, eight loads in flight (rows begin on 128-byte boundaries, and their pitch is
+  // a multiple of 32 samples: a load that straddles the row's end stays inside it)
+  constexpr int V = 16 / static_cast<int>(sizeof(T));
+  struct alignas(16) Vec {
+    T e[V];
+  };
+  T* to = tile + 33 * ((V * lane) >> 5) + ((V * lane) & 31);
+#pragma unroll 1
+  for (int k0 = 0; k0 < 32 / V; k0 += 8) {
+    if (32 * V * k0 >= left) break;
+    Vec v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int32_t i = V * (32 * (k0 + k) + lane);
+      if (i < left) v[k] = *reinterpret_cast<const Vec*>(row + i0 + i);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int32_t i = V * (32 * (k0 + k) + lane);
+      if (32 * V * (k0 + k) < left) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) to[33 * V * (k0 + k) + e] = i + e < left ? v[k].e[e] : T(0);
+      }
+    }
   }
   __syncwarp();
   double acc = 0.0;
@@ -99,8 +119,10 @@ __device__ __forceinline__ double row_step(const T* __restrict__ row, int32_t n,
   return warp_tree32(acc);
 }
 
-// Rows of one step: a warp per row. Longer rows (per_row): a CTA per row, its warps over the steps (one
-// warp walked all 20 steps of a 20 011-sample line in 54 us).
+// Rows of one step: a warp per row. Longer rows (per_row): a CTA per row, its warps over the steps. Bound by
+// the loads' latency (with scalar loads 8 % of the DRAM's rate, 13 of 15 stalled warps on a load): 64 images
+// of 512 x 512 float32 63 -> 26 us, 4 volumes of 256^3 316 -> 167 us, a line of 20 011 float64 samples 45
+// -> 13 us (54 us by one warp).
 constexpr int kMaxSteps = 128;
 template <class T>
 constexpr int kRowThreads = 1024 / static_cast<int>(sizeof(T));  // (the tiles of 8 float or 4 double warps: 34 KB)
