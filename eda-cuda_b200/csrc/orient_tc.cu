@@ -11,20 +11,20 @@
 // cuFFT in float32, cpp/src/method/orientation.cu:674-767 of eda-cuda.) The basis is split once on
 // the host; the field tile is split in shared memory after its TMA load.
 //
-// Kernel (persistent: one CTA of 320 threads per SM runs 128 x 128 output tiles in turn):
-//   warp 4      TMA producer: A tile (128 rows x 32 floats, 128B swizzle) and the hi and lo basis
-//               tiles per k-block into a 3-stage ring (full / empty mbarriers);
-//   warps 0-3   split the A tile into hi and lo tiles (3xTF32: hi in place, 128B swizzle; BF16x3:
-//               two bfloat16 tiles of 64-byte rows in the 64B swizzle), fence the async proxy,
-//               arrive on the stage's split barrier;
-//   warp 5      allocates 256 TMEM columns, two accumulators; one thread issues the split MMAs of
-//               every k-block (3 x 4 kind::tf32 with K = 8, or 3 x 2 kind::f16 with K = 16; M = N =
-//               128), commits each stage back to the producer and each tile to the epilogue;
+// Kernel (persistent: one CTA of 320 threads per SM runs tiles of 128 rows and 128 or 256 columns in turn):
+//   warp 4      TMA producer: A tile (128 rows) and the hi and lo basis tiles per k-block into a ring of
+//               3 or 4 stages (full / empty mbarriers);
+//   warps 0-3   split the A tile into hi and lo tiles (3xTF32: hi in place; BF16x3: two bfloat16 tiles),
+//               fence the async proxy, arrive on the stage's split barrier;
+//   warp 5      allocates two accumulators in TMEM; one thread issues the split MMAs of every k-block
+//               (kind::tf32 with K = 8, or kind::f16 with K = 16), commits each stage back to the producer
+//               and each tile to the epilogue;
 //   warps 6-9   the epilogue: tcgen05.ld of their TMEM lane quarter and the transposed store, while
 //               the next tile's products go to the other accumulator.
-// Bound by shared-memory bandwidth: the MMAs read 8 KB of operands each, and every k-block is written by
-// TMA, read and written by the split. 16 fields of 1000 x 768: 138 us per pass (154 us with one tile
-// per CTA, whose set-up, pipeline fill and epilogue stood in a row with its MMAs).
+// Bound by the MMAs' and the k-blocks' fixed costs (tensor pipe 40 % active at N = 128, L2 15 %): the split
+// A in tensor memory with four stages (129 us against 138 for 16 fields of 1000 x 768), 256 rows per tile
+// (139), descriptors stepped by additions (135), the rounding by integer operations (no change) and
+// k-blocks of 16 in six stages (154) were tried at N = 128; N = 256 takes 101.
 // The store writes the tile transposed: the transformed axis becomes the slowest axis of the
 // element and the next axis the contiguous one (a rotation of the layout), so every transform of
 // the orientation reads K-major rows, and D passes bring a field back to its layout.
@@ -41,49 +41,51 @@
 namespace edab {
 namespace tc {
 
-constexpr int kBM = 128, kBN = 128, kBK = 32, kStages = 3;
+constexpr int kBM = 128;
 constexpr int kThreadsTc = 320;
 constexpr unsigned long long kWaitNs = 2000000000ull;
 
-// The stage layout of a split mode. 3xTF32: [A hi (TMA, then split in place) | A lo | B hi | B lo],
-// 16 KiB each, rows of 128 bytes. BF16x3: [A float32 (TMA) 16 KiB | A hi | A lo | B hi | B lo], the
-// bfloat16 tiles 8 KiB each, rows of 64 bytes. Every tile starts on a 1024-byte boundary.
-template <bool BF16>
+// The stage layout of a split mode and tiles of BN columns. 3xTF32: [A hi (TMA, then split in place) | A lo |
+// B hi | B lo], rows of 32 floats (BN = 128) or 16 (BN = 256: two stages of 32 were too few); BF16x3:
+// [A float32 (TMA), rows of 128 bytes | A hi | A lo | B hi | B lo], rows of 32 bfloat16. Every tile starts
+// on a 1024-byte boundary; its swizzle spans a row.
+template <bool BF16, int BN>
 struct Stage {
-  static constexpr int kTileF32 = kBM * kBK * 4;                      // 16 KiB: the float32 A tile
-  static constexpr int kTileOp = BF16 ? kBM * kBK * 2 : kBM * kBK * 4;  // one operand tile
+  static_assert(!BF16 || BN == 128);
+  static constexpr int kBK = BN == 256 ? 16 : 32;
+  static constexpr int kStages = BN == 256 ? 4 : 3;
+  static constexpr int kRowBytes = kBK * (BF16 ? 2 : 4);  // of an operand tile
+  static constexpr int kTileF32 = kBM * kBK * 4;  // the float32 A tile
+  static constexpr int kTileA = kBM * kRowBytes, kTileB = BN * kRowBytes;
   static constexpr int kAhi = BF16 ? kTileF32 : 0;
-  static constexpr int kAlo = kAhi + kTileOp;
-  static constexpr int kBhi = kAlo + kTileOp;
-  static constexpr int kBlo = kBhi + kTileOp;
-  static constexpr int kBytes = kBlo + kTileOp;
-  static constexpr int kTmaBytes = kTileF32 + 2 * kTileOp;  // A float32, B hi, B lo
+  static constexpr int kAlo = kAhi + kTileA;
+  static constexpr int kBhi = kAlo + kTileA;
+  static constexpr int kBlo = kBhi + kTileB;
+  static constexpr int kBytes = kBlo + kTileB;
+  static constexpr int kTmaBytes = kTileF32 + 2 * kTileB;  // A float32, B hi, B lo
   static constexpr int kSmem = kStages * kBytes + 1024 + 256;
 };
 
 // Instruction descriptors (D float32, both operands K-major, N, M): kind::tf32 with tf32 A and B;
 // kind::f16 with bfloat16 A and B.
-constexpr uint32_t kIdescTf32 = (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(kBN >> 3) << 17) |
+template <int BN>
+constexpr uint32_t kIdescTf32 = (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) |
                                 (static_cast<uint32_t>(kBM >> 4) << 24);
-constexpr uint32_t kIdescBf16 = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kBN >> 3) << 17) |
+template <int BN>
+constexpr uint32_t kIdescBf16 = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) |
                                 (static_cast<uint32_t>(kBM >> 4) << 24);
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-// Shared-memory matrix descriptor of a K-major tile with the 128-byte swizzle: rows of 128 bytes,
-// 8-row groups 1024 bytes apart (SBO), version 1, layout SWIZZLE_128B.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
+// Shared-memory matrix descriptor of a K-major tile with rows of 128 or 64 bytes and the swizzle of that
+// span: 8-row groups 1024 or 512 bytes apart (SBO), version 1, layout SWIZZLE_128B or SWIZZLE_64B.
+template <int ROW_BYTES>
+__device__ __forceinline__ uint64_t sw_desc(uint32_t addr) {
+  static_assert(ROW_BYTES == 128 || ROW_BYTES == 64);
   return static_cast<uint64_t>((addr >> 4) & 0x3fffu) | (static_cast<uint64_t>(1) << 16) |
-         (static_cast<uint64_t>(1024 >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
-         (static_cast<uint64_t>(2) << 61);
-}
-// The same for a K-major tile with the 64-byte swizzle: rows of 64 bytes, 8-row groups 512 bytes
-// apart, layout SWIZZLE_64B.
-__device__ __forceinline__ uint64_t sw64_desc(uint32_t addr) {
-  return static_cast<uint64_t>((addr >> 4) & 0x3fffu) | (static_cast<uint64_t>(1) << 16) |
-         (static_cast<uint64_t>(512 >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
-         (static_cast<uint64_t>(4) << 61);
+         (static_cast<uint64_t>(8 * ROW_BYTES >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
+         (static_cast<uint64_t>(ROW_BYTES == 128 ? 2 : 4) << 61);
 }
 __device__ __forceinline__ unsigned long long now_ns() {
   unsigned long long t;
@@ -130,20 +132,22 @@ __device__ __forceinline__ float to_tf32(float x) {
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
   return __uint_as_float(r);
 }
+template <int BN>
 __device__ __forceinline__ void mma_tf32(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-      "l"(adesc), "l"(bdesc), "r"(kIdescTf32), "r"(accumulate)
+      "l"(adesc), "l"(bdesc), "r"(kIdescTf32<BN>), "r"(accumulate)
       : "memory");
 }
+template <int BN>
 __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-      "l"(adesc), "l"(bdesc), "r"(kIdescBf16), "r"(accumulate)
+      "l"(adesc), "l"(bdesc), "r"(kIdescBf16<BN>), "r"(accumulate)
       : "memory");
 }
 // bfloat16 of x rounded to nearest even, as raw bits (x finite or infinite; NaN stays NaN).
@@ -196,11 +200,12 @@ __device__ __forceinline__ bool tile_runs(const RotOut& ro, const int32_t* __res
   return false;
 }
 
-template <bool BF16>
+template <bool BF16, int BN>
 __global__ void __launch_bounds__(kThreadsTc, 1)
     gemm_tc(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, RotOut ro,
             float* __restrict__ out, const int32_t* __restrict__ run, int32_t* __restrict__ err) {
-  using L = Stage<BF16>;
+  using L = Stage<BF16, BN>;
+  constexpr int kStages = L::kStages, kBK = L::kBK;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + kStages * L::kBytes);
@@ -227,7 +232,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
   __syncthreads();
   if (warp == 5) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(2 * kBN)
+                 "r"(2 * BN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
       uint32_t it = 0;
       for (int64_t t = blockIdx.x; ok && t < ro.tiles; t += gridDim.x) {
         const int64_t m0 = t / ro.n_tiles * kBM;
-        const int32_t n0 = static_cast<int32_t>(t % ro.n_tiles) * kBN;
+        const int32_t n0 = static_cast<int32_t>(t % ro.n_tiles) * BN;
         if (!tile_runs(ro, run, m0)) continue;
         for (int32_t kb = 0; kb < ro.kblocks; ++kb, ++it) {
           const int s = static_cast<int>(it % kStages);
@@ -269,7 +274,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
       for (int64_t t = blockIdx.x; ok && t < ro.tiles; t += gridDim.x) {
         if (!tile_runs(ro, run, t / ro.n_tiles * kBM)) continue;
         const int buf = static_cast<int>(j & 1u);
-        const uint32_t acc = tmem + static_cast<uint32_t>(buf * kBN);
+        const uint32_t acc = tmem + static_cast<uint32_t>(buf * BN);
         if (!mbar_wait(acc_empty(buf), ((j >> 1) & 1u) ^ 1u)) {  // the epilogue has read it
           ok = false;
           break;
@@ -287,17 +292,17 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
 #pragma unroll
             for (int kk = 0; kk < kBK / 16; ++kk) {
               const uint32_t off = kk * 32;  // 16 bfloat16 of K inside the 64-byte swizzled row
-              mma_bf16(acc, sw64_desc(a_hi + off), sw64_desc(b_hi + off), (kb | kk) != 0);
-              mma_bf16(acc, sw64_desc(a_hi + off), sw64_desc(b_lo + off), 1u);
-              mma_bf16(acc, sw64_desc(a_lo + off), sw64_desc(b_hi + off), 1u);
+              mma_bf16<BN>(acc, sw_desc<L::kRowBytes>(a_hi + off), sw_desc<L::kRowBytes>(b_hi + off), (kb | kk) != 0);
+              mma_bf16<BN>(acc, sw_desc<L::kRowBytes>(a_hi + off), sw_desc<L::kRowBytes>(b_lo + off), 1u);
+              mma_bf16<BN>(acc, sw_desc<L::kRowBytes>(a_lo + off), sw_desc<L::kRowBytes>(b_hi + off), 1u);
             }
           } else {
 #pragma unroll
             for (int kk = 0; kk < kBK / 8; ++kk) {
-              const uint32_t off = kk * 32;  // 8 tf32 of K inside the 128-byte swizzled row
-              mma_tf32(acc, sw128_desc(a_hi + off), sw128_desc(b_hi + off), (kb | kk) != 0);
-              mma_tf32(acc, sw128_desc(a_hi + off), sw128_desc(b_lo + off), 1u);
-              mma_tf32(acc, sw128_desc(a_lo + off), sw128_desc(b_hi + off), 1u);
+              const uint32_t off = kk * 32;  // 8 tf32 of K inside the swizzled row
+              mma_tf32<BN>(acc, sw_desc<L::kRowBytes>(a_hi + off), sw_desc<L::kRowBytes>(b_hi + off), (kb | kk) != 0);
+              mma_tf32<BN>(acc, sw_desc<L::kRowBytes>(a_hi + off), sw_desc<L::kRowBytes>(b_lo + off), 1u);
+              mma_tf32<BN>(acc, sw_desc<L::kRowBytes>(a_lo + off), sw_desc<L::kRowBytes>(b_hi + off), 1u);
             }
           }
           mma_commit(empty_bar(s));
@@ -369,7 +374,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
     uint32_t j = 0;
     for (int64_t t = blockIdx.x; ok && t < ro.tiles; t += gridDim.x) {
       const int64_t m0 = t / ro.n_tiles * kBM;
-      const int32_t n0 = static_cast<int32_t>(t % ro.n_tiles) * kBN;
+      const int32_t n0 = static_cast<int32_t>(t % ro.n_tiles) * BN;
       if (!tile_runs(ro, run, m0)) continue;
       const int buf = static_cast<int>(j & 1u);
       // the tcgen05.ld below is warp-collective: the warp decides together
@@ -388,9 +393,9 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
         obase = b * ro.f_out + hi * ro.pitch_out + lo;
       }
 #pragma unroll 1
-      for (int c = 0; c < kBN / 32; ++c) {
+      for (int c = 0; c < BN / 32; ++c) {
         float v[32];
-        tmem_ld32(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * kBN + c * 32), v);
+        tmem_ld32(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * BN + c * 32), v);
         if (valid) {
 #pragma unroll
           for (int jj = 0; jj < 32; ++jj) {
@@ -409,7 +414,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
   __syncthreads();
   if (warp == 5) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kBN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
   }
 }
 
@@ -433,19 +438,19 @@ EncodeTiled encode_fn() {
   return fn;
 }
 
-// A 2-D tensor map of float32 (128-byte swizzle) or bfloat16 (64-byte swizzle) elements: inner
-// extent `inner` (contiguous), `outer` rows `stride` elements apart, boxes of 32 x box_rows
-// elements (one swizzled row each); reads past the extents return zeros.
-CUtensorMap make_map(const void* base, bool bf16, uint64_t inner, uint64_t outer, uint64_t stride, uint32_t box_rows) {
+// A 2-D tensor map of float32 or bfloat16 elements: inner extent `inner` (contiguous), `outer` rows
+// `stride` elements apart, boxes of box_k x box_rows elements, a swizzled row of 64 or 128 bytes each; reads
+// past the extents return zeros.
+CUtensorMap make_map(const void* base, bool bf16, uint64_t inner, uint64_t outer, uint64_t stride, int box_k, int box_rows) {
   CUtensorMap m;
   std::memset(&m, 0, sizeof m);
   const cuuint64_t dims[2] = {inner, outer};
   const cuuint64_t strides[1] = {stride * (bf16 ? 2 : 4)};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kBK), box_rows};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_k), static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = encode_fn()(&m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
                                  const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                 bf16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                                 box_k * (bf16 ? 2 : 4) == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     throw CudaError("eda: cuTensorMapEncodeTiled failed (" + std::to_string(static_cast<int>(r)) + ")",
@@ -454,11 +459,23 @@ CUtensorMap make_map(const void* base, bool bf16, uint64_t inner, uint64_t outer
   return m;
 }
 
-template <bool BF16>
-void set_smem_once() {
-  once_on_device(reinterpret_cast<const void*>(gemm_tc<BF16>), [] {
-    EDAB_CUDA(cudaFuncSetAttribute(gemm_tc<BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, Stage<BF16>::kSmem));
+template <bool BF16, int BN>
+void launch(cudaStream_t s, const RotPass& p, const void* basis, int32_t kpad, int32_t npad, const float* in, float* out,
+            const int32_t* run, int32_t* err, RotOut ro, int sms) {
+  using L = Stage<BF16, BN>;
+  const CUtensorMap ta = make_map(in, false, static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.M),
+                                  static_cast<uint64_t>(p.pitch_in), L::kBK, kBM);
+  const CUtensorMap tb = make_map(basis, BF16, static_cast<uint64_t>(kpad), static_cast<uint64_t>(2 * npad),
+                                  static_cast<uint64_t>(kpad), L::kBK, BN);
+  ro.kblocks = (p.K + L::kBK - 1) / L::kBK;
+  ro.n_tiles = (p.K + BN - 1) / BN;
+  ro.tiles = (p.M + kBM - 1) / kBM * ro.n_tiles;
+  once_on_device(reinterpret_cast<const void*>(gemm_tc<BF16, BN>), [] {
+    EDAB_CUDA(cudaFuncSetAttribute(gemm_tc<BF16, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmem));
   });
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(ro.tiles, sms));
+  gemm_tc<BF16, BN><<<grid, kThreadsTc, L::kSmem, s>>>(ta, tb, ro, out, run, err);
+  EDAB_LAUNCH("gemm_tc");
 }
 
 }  // namespace tc
@@ -467,34 +484,28 @@ void set_smem_once() {
 void rot_pass_tc(cudaStream_t s, const RotPass& p, const void* basis, bool bf16, int32_t kpad, int32_t npad,
                  const float* in, float* out, const int32_t* run, int32_t* err) {
   if (p.M < 1) return;
-  const CUtensorMap ta = tc::make_map(in, false, static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.M),
-                                      static_cast<uint64_t>(p.pitch_in), tc::kBM);
-  const CUtensorMap tb = tc::make_map(basis, bf16, static_cast<uint64_t>(kpad), static_cast<uint64_t>(2 * npad),
-                                      static_cast<uint64_t>(kpad), tc::kBN);
   tc::RotOut ro{};
   ro.M = p.M;
   ro.N = p.K;
-  ro.kblocks = (p.K + tc::kBK - 1) / tc::kBK;
   ro.npad = npad;
   ro.rows = p.rows;
   ro.n_lo = p.n_lo;
   ro.pitch_out = p.pitch_out;
   ro.s_j = p.s_j;
   ro.f_out = p.f_out;
-  ro.n_tiles = (p.K + tc::kBN - 1) / tc::kBN;
-  ro.tiles = (p.M + tc::kBM - 1) / tc::kBM * ro.n_tiles;
   int sms = 148, dev = 0;
   EDAB_CUDA(cudaGetDevice(&dev));
   EDAB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const dim3 grid(static_cast<unsigned>(std::min<int64_t>(ro.tiles, sms)));
-  if (bf16) {
-    tc::set_smem_once<true>();
-    tc::gemm_tc<true><<<grid, tc::kThreadsTc, tc::Stage<true>::kSmem, s>>>(ta, tb, ro, out, run, err);
-  } else {
-    tc::set_smem_once<false>();
-    tc::gemm_tc<false><<<grid, tc::kThreadsTc, tc::Stage<false>::kSmem, s>>>(ta, tb, ro, out, run, err);
-  }
-  EDAB_LAUNCH("gemm_tc");
+  // Tiles of 256 columns take half the MMAs (at M = 128 one of N = 256 runs in 1.5 times one of N = 128) and
+  // half the reads of A: 16 fields of 1000 x 768 101 us per pass (138 with 128 columns), 64 of 512 x 512 88
+  // us (102). While the tiles of 128 fit the SMs at once, the shorter tiles win: one field of 301 x 443 16 us
+  // (22 with 256). So: by the waves, a wide tile counted 1.5.
+  const auto waves = [&](int64_t bn) { return ((p.M + tc::kBM - 1) / tc::kBM * ((p.K + bn - 1) / bn) + sms - 1) / sms; };
+  const bool w = 3 * waves(256) <= 2 * waves(128);
+  const auto go = [&](auto launch) { launch(s, p, basis, kpad, npad, in, out, run, err, ro, sms); };
+  if (bf16) go(tc::launch<true, 128>);
+  else if (w) go(tc::launch<false, 256>);
+  else go(tc::launch<false, 128>);
 }
 
 }  // namespace edab
