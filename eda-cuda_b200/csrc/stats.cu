@@ -576,6 +576,217 @@ __global__ void __launch_bounds__(TH) select_cluster(Geom g, SelView<T> a, const
   }
 }
 
+// The small form: one CTA per element whose keys fit its shared memory. The keys are gathered densely with
+// their smallest and largest; a histogram of 2048 bins over the range that is left finds the bin of both
+// ranks (neighbours or the same), until few keys are left (ranked by comparing them all), the ranks part
+// (the lower bin's largest key, the upper one's smallest) or a bin is one key. Bound by the gather's loads
+// and the barriers: no digit of the keys is fixed, so one histogram mostly does. (In clusters a median of
+// 4096 samples took three passes of 11 fixed digits, 25 us at 64 signals; 7 us here.)
+constexpr int kSmallBins = 2048, kSmallList = 128, kSmallThreads = 1024;
+constexpr int64_t kSmallItems = 32768;
+constexpr size_t kSmallBytes = 216 * 1024;  // (the state takes 3 KB more)
+template <class K>
+struct SmallState {
+  K lo, hi, v0, v1;
+  unsigned n, r0, r1, d0, d1, listed;
+  unsigned warp_tot[kSmallThreads / 32];
+  K list[kSmallList];
+};
+__device__ __forceinline__ int bit_length(uint32_t v) { return 32 - __clz(static_cast<int>(v)); }
+__device__ __forceinline__ int bit_length(uint64_t v) { return 64 - __clzll(static_cast<long long>(v)); }
+template <class K>
+__device__ __forceinline__ K warp_max_key(K v) {
+  if constexpr (sizeof(K) == 4) return __reduce_max_sync(0xffffffffu, v);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const K o = __shfl_xor_sync(0xffffffffu, v, d);
+    v = o > v ? o : v;
+  }
+  return v;
+}
+__device__ __forceinline__ void shared_max(uint32_t* at, uint32_t v) { atomicMax(at, v); }
+__device__ __forceinline__ void shared_max(uint64_t* at, uint64_t v) {
+  atomicMax(reinterpret_cast<unsigned long long*>(at), static_cast<unsigned long long>(v));
+}
+// The element's largest of v over the CTA goes to *at (set before the last barrier).
+template <class K>
+__device__ __forceinline__ void block_max(K* at, K v) {
+  v = warp_max_key(v);
+  if ((threadIdx.x & 31) == 0) shared_max(at, v);
+}
+
+// dynamic shared memory: the keys [items], the bins
+template <class T, class K>
+__global__ void __launch_bounds__(kSmallThreads) select_small(Geom g, SelView<T> a, const int32_t* run, double q, double* out,
+                                                     int64_t* count_out) {
+  extern __shared__ __align__(16) unsigned char sel_smem[];
+  __shared__ SmallState<K> st;
+  const int64_t b = blockIdx.x;
+  if (run && !run[b]) return;
+  auto* bins = reinterpret_cast<uint32_t*>(sel_smem);
+  K* keys = reinterpret_cast<K*>(bins + kSmallBins);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, TH = blockDim.x;
+  if (tid == 0) {
+    st.lo = st.hi = K(0);  // lo: the complements' largest, for now
+    st.n = 0;
+  }
+  __syncthreads();
+  {
+    K top = K(0), bottom = K(0);
+    const int32_t items = static_cast<int32_t>(a.items);
+    for (int32_t t0 = 0; t0 < items; t0 += 4 * TH) {
+      K k[4];
+      bool have[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int32_t t = t0 + u * TH + tid;
+        k[u] = K(0);
+        have[u] = t < items && sel_key_of<T, K>(g, a, b, t, &k[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const unsigned m = __ballot_sync(0xffffffffu, have[u]);
+        if (!m) continue;
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(&st.n, static_cast<unsigned>(__popc(m)));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (have[u]) {
+          keys[base + __popc(m & ((1u << lane) - 1u))] = k[u];
+          top = k[u] > top ? k[u] : top;
+          const K c = static_cast<K>(~k[u]);
+          bottom = c > bottom ? c : bottom;
+        }
+      }
+    }
+    block_max(&st.hi, top);
+    block_max(&st.lo, bottom);
+  }
+  __syncthreads();
+  const int32_t n = static_cast<int32_t>(st.n);
+  if (n == 0) {
+    if (tid == 0) {
+      out[b] = d_nan();
+      if (count_out) count_out[b] = 0;
+    }
+    return;
+  }
+  K lo = static_cast<K>(~st.lo), hi = st.hi;
+  unsigned r0, r1;
+  double gamma = 0.0;
+  if (q < 0) {
+    r0 = static_cast<unsigned>((n - 1) / 2);
+    r1 = static_cast<unsigned>(n / 2);
+  } else {
+    long long i = 0, j = 0;
+    linear_index(n, q, &i, &j, &gamma);
+    r0 = static_cast<unsigned>(i);
+    r1 = static_cast<unsigned>(j);
+  }
+  unsigned left = static_cast<unsigned>(n);  // keys in [lo, hi]; the ranks count from lo's
+  K v0 = K(0), v1 = K(0);
+  for (;;) {  // (the range shrinks to a bin, 2^-10 of it or less, each time)
+    if (lo == hi) {
+      v0 = v1 = lo;
+      break;
+    }
+    if (left <= kSmallList) {
+      if (tid == 0) st.listed = 0;
+      __syncthreads();
+      for (int32_t i = tid; i < n; i += TH) {
+        const K k = keys[i];
+        if (k >= lo && k <= hi) st.list[atomicAdd(&st.listed, 1u)] = k;
+      }
+      __syncthreads();
+      if (tid < static_cast<int>(left)) {
+        const K mine = st.list[tid];
+        unsigned rank = 0;
+        for (int i = 0; i < static_cast<int>(left); ++i) {
+          const K k = st.list[i];
+          rank += (k < mine || (k == mine && i < tid)) ? 1u : 0u;
+        }
+        if (rank == r0) st.v0 = mine;
+        if (rank == r1) st.v1 = mine;
+      }
+      __syncthreads();
+      v0 = st.v0;
+      v1 = st.v1;
+      break;
+    }
+    const int shift = max(bit_length(static_cast<K>(hi - lo)) - 11, 0);
+    for (int i = tid; i < kSmallBins; i += TH) bins[i] = 0u;
+    if (tid == 0) st.v0 = st.v1 = K(0);
+    __syncthreads();
+    const int32_t end = (n + 31) / 32 * 32;
+    for (int32_t i = tid; i < end; i += TH) {
+      const K k = i < n ? keys[i] : K(0);
+      count_digit(bins, static_cast<uint32_t>((k - lo) >> shift), i < n && k >= lo && k <= hi);
+    }
+    __syncthreads();
+    // the bins of the ranks: exclusive prefix sums over kSmallBins / TH consecutive bins per thread
+    const int per = kSmallBins / TH;
+    unsigned mine = 0;
+    for (int i = 0; i < per; ++i) mine += bins[tid * per + i];
+    unsigned incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const unsigned o = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += o;
+    }
+    if (lane == 31) st.warp_tot[warp] = incl;
+    __syncthreads();
+    unsigned before = incl - mine;
+    for (int w = 0; w < warp; ++w) before += st.warp_tot[w];
+    for (int i = 0; i < per; ++i) {
+      const unsigned c = bins[tid * per + i];
+      if (r0 >= before && r0 < before + c) {
+        st.d0 = static_cast<unsigned>(tid * per + i);
+        st.r0 = r0 - before;
+        st.listed = c;
+      }
+      if (r1 >= before && r1 < before + c) {
+        st.d1 = static_cast<unsigned>(tid * per + i);
+        st.r1 = r1 - before;
+      }
+      before += c;
+    }
+    __syncthreads();
+    const K d0 = st.d0, d1 = st.d1;
+    if (shift == 0) {
+      v0 = lo + d0;
+      v1 = lo + d1;
+      break;
+    }
+    if (d0 != d1) {  // neighbours in rank: the lower bin's largest key and the upper one's smallest
+      K low = K(0), up = K(0);
+      for (int32_t i = tid; i < n; i += TH) {
+        const K k = keys[i];
+        if (k < lo || k > hi) continue;
+        const K d = (k - lo) >> shift;
+        if (d == d0) low = k > low ? k : low;
+        if (d == d1) up = static_cast<K>(~k) > up ? static_cast<K>(~k) : up;
+      }
+      __syncwarp();
+      block_max(&st.v0, low);
+      block_max(&st.v1, up);
+      __syncthreads();
+      v0 = st.v0;
+      v1 = static_cast<K>(~st.v1);
+      break;
+    }
+    r0 = st.r0;
+    r1 = st.r1;
+    left = st.listed;
+    lo = lo + (d0 << shift);
+    if (hi - lo >= (K(1) << shift)) hi = lo + ((K(1) << shift) - 1);
+    __syncthreads();  // the state is read before the next round writes it
+  }
+  if (tid == 0) {
+    const double x0 = key_value(v0), x1 = key_value(v1);
+    out[b] = q < 0 ? ((n & 1) ? x0 : __dmul_rn(__dadd_rn(x0, x1), 0.5)) : linear_between(x0, x1, gamma);
+    if (count_out) count_out[b] = n;
+  }
+}
+
 // The grid-wide form for batches of few, large elements (select):
 // per digit, a launch over many CTAs per element (warp-aggregated shared-memory counts, flushed with
 // one global atomic per digit value and CTA) whose last CTA finds the digit by the same block-wide
@@ -1107,11 +1318,10 @@ void select(cudaStream_t s, const Geom& g, const Sel<T>& sel, double q, const in
     a.items = static_cast<int64_t>(a.naxes) * g.field;
   }
   if (g.batch > 65535) throw std::invalid_argument("edab: select batch too large");
-  // Clusters (one launch): of 256-thread CTAs when the batch fills the GPU with them, else of
-  // 1024-thread CTAs while an element has at most 8 items for each of their threads (a median of 2048
-  // samples: 13 us and one launch, against 8 launches of 3 us); larger elements of small batches take
-  // the grid-wide form, a launch per digit over many CTAs (133 000 items: 40 us, against 54 us in one
-  // cluster).
+  // Otherwise clusters (one launch): of 256-thread CTAs when the batch fills the GPU with them, else of
+  // 1024-thread CTAs while an element has at most 8 items for each of their threads; larger elements of
+  // small batches take the grid-wide form, a launch per digit over many CTAs (133 000 items: 26 us for
+  // 32-bit keys, against 54 us in one cluster).
   int sms = 148;
   {
     int dev = 0;
@@ -1128,6 +1338,28 @@ void select(cudaStream_t s, const Geom& g, const Sel<T>& sel, double q, const in
       }
     }
     if (!done) run = select_split<T, uint64_t>(s, g, a, q, run, out, count, scratch, sms);
+  }
+  // Elements whose keys fit one CTA's shared memory: the small form (medians of 2048 samples 5.8 us, of up to
+  // 8192 in batches 7 to 12 us, of 20 011 float64 samples 21 us; as clusters 12.5, 25 to 33 and 30 us).
+  const bool narrow = std::is_same_v<T, float> && sel.center == nullptr;  // 32-bit keys
+  const size_t small = static_cast<size_t>(a.items) * (narrow ? 4 : 8) + kSmallBins * sizeof(uint32_t);
+  if (a.items <= kSmallItems && small <= kSmallBytes) {
+    const unsigned th = a.items > 4096 ? 1024u : a.items > 2048 ? 512u : a.items > 512 ? 256u : 128u;
+    const auto go = [&](auto kernel) {
+      once_on_device(reinterpret_cast<const void*>(kernel), [&] {
+        EDAB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmallBytes)));
+      });
+      kernel<<<static_cast<unsigned>(g.batch), th, small, s>>>(g, a, run, q, out, count);
+      EDAB_LAUNCH("select_small");
+    };
+    if constexpr (std::is_same_v<T, float>) {
+      if (narrow) {
+        go(select_small<T, uint32_t>);
+        return;
+      }
+    }
+    go(select_small<T, uint64_t>);
+    return;
   }
   const bool many = g.batch * kSelClusterMax >= 2 * static_cast<int64_t>(sms);
   if (!kSelClusters || (!many && a.items > int64_t{kSelClusterMax} * kSelWide * 8)) {
