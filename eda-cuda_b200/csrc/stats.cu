@@ -264,7 +264,8 @@ constexpr int kDigitBins = 1 << kDigitBits;
 constexpr int kSelClusterMax = 8;
 // Items of an element (at least, at most) and of the batch that the split form takes: its list of 8 % is
 // selected from by one CTA per element, which at 50 M items took 8.7 ms (the grid-wide form 2.9 ms).
-constexpr int64_t kSplitItems = 65536, kSplitMost = int64_t{1} << 22, kSplitTotal = int64_t{1} << 21;
+// Batches of fewer elements leave the GPU to that CTA (one element of 2 M items: 0.5 ms).
+constexpr int64_t kSplitItems = 65536, kSplitMost = int64_t{1} << 22, kSplitTotal = int64_t{1} << 21, kSplitBatch = 16;
 constexpr int kSelWide = 1024;  // threads of a cluster's CTA in a small batch
 // The cluster form for batches that fill the GPU with clusters (1), or the grid-wide form always (0).
 #ifndef EDAB_SEL_CLUSTERS
@@ -1329,7 +1330,8 @@ void select(cudaStream_t s, const Geom& g, const Sel<T>& sel, double q, const in
     EDAB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   }
   // Many items: the split form first, then the others for the elements that it hands on.
-  if (scratch && a.items >= kSplitItems && a.items <= kSplitMost && a.items * g.batch >= kSplitTotal) {
+  if (scratch && a.items >= kSplitItems && a.items <= kSplitMost && g.batch >= kSplitBatch &&
+      a.items * g.batch >= kSplitTotal) {
     bool done = false;
     if constexpr (std::is_same_v<T, float>) {
       if (sel.center == nullptr) {
