@@ -208,7 +208,8 @@ EDA_API int eda_pointer_device(const void* p, int* device);
 
 /* The cube passes' autotuner (no counterpart in the reference, whose launch shapes are fixed,
  * cpp/src/field/vhgw.cu:540-559). eda_autotune times the candidate launch shapes of the cube passes
- * (lines per CTA; a record's other two numbers are kept and have no effect) on a synthetic field of the geometry (dtype, dim, batch, n) on the current device, records the
+ * (lines per CTA; a record's other two numbers are kept and have no effect) on a synthetic field of
+ * the geometry (dtype, dim, batch, n) on the current device, records the
  * fastest for that geometry (results are bit-identical under every shape) and, with cache_path,
  * writes every record to that text file; report receives a JSON summary. eda_tuning_load reads a
  * cache file into the records (the environment variable EDA_TUNING_CACHE names one that the first
