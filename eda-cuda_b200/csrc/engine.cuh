@@ -186,6 +186,7 @@ struct Ctl {
   double sqrt2;       // sqrt(2) correctly rounded
   double powq[48];    // sqrt(2)^j for j = -8 .. 39 (host pow): ladder and G2 rungs, index j + 8
   int32_t max_imf, check_finite, rows_cap;
+  int32_t product;    // the float32 transforms' product (TransformPrecision) when the call began
 };
 Ctl make_ctl(const Geom& g, bool f32, int32_t sifts, double tau, int32_t max_imf, bool check_finite,
              int32_t rows_cap);

@@ -114,6 +114,7 @@ Ctl make_ctl(const Geom& g, bool f32, int32_t sifts, double tau, int32_t max_imf
   c.max_imf = max_imf;
   c.check_finite = check_finite ? 1 : 0;
   c.rows_cap = rows_cap;
+  c.product = static_cast<int32_t>(transform_precision());
   return c;
 }
 
@@ -678,7 +679,7 @@ class Engine {
     const auto put = [&](const auto& v) { key.append(reinterpret_cast<const char*>(&v), sizeof v); };
     const CubeTune tune = cube_tune_for(g_, 0, sizeof(T));
     const int32_t ints[] = {part, count, static_cast<int32_t>(sizeof(T)), g_.dim, g_.n[0], g_.n[1], g_.n[2],
-                            static_cast<int32_t>(transform_precision()), tune.lines, c_.sifts, c_.check_finite, c_.max_imf, c_.rows_cap};
+                            c_.product, tune.lines, c_.sifts, c_.check_finite, c_.max_imf, c_.rows_cap};
     put(ints);
     put(g_.batch);
     put(c_.tau);
@@ -1110,7 +1111,7 @@ void Engine<T>::orientation_and_build() {
   int32_t* mask_s = mask_;
   const int64_t B = B_;
   if (g_.dim >= 2) {
-    orientation<T>(s_, g_, *plan_, r_, el_, on, n_, coh_, owork_, c_.two_sigma2, any_ + kTcErr);
+    orientation<T>(s_, g_, *plan_, static_cast<TransformPrecision>(c_.product), r_, el_, on, n_, coh_, owork_, c_.two_sigma2, any_ + kTcErr);
     for_elements(s_, B_, [=] __device__(int64_t b) {
       if (el[b].status == kActive && el[b].nonfinite) fail2(el[b], win_s, mask_s, B, b);
     });

@@ -86,6 +86,7 @@ void run_monogenic(const void* x, bool on_device, int dim, int64_t batch, const 
   while (Bc > 1 && need(Bc) + margin > free_b) Bc = (Bc + 1) / 2;
   ws.reserve(need(Bc), s);
   const OrientPlan& plan = orient_plan(g, std::is_same_v<T, double>);
+  const TransformPrecision product = transform_precision();
   std::vector<int32_t> bad(static_cast<size_t>(Bc));
   for (int64_t b0 = 0; b0 < batch; b0 += Bc) {
     const int64_t nb = std::min(Bc, batch - b0);
@@ -116,7 +117,7 @@ void run_monogenic(const void* x, bool on_device, int dim, int64_t batch, const 
     EDAB_LAUNCH("field_max");
     prescale<T><<<grid, kThreads, 0, s>>>(gc, amax, exp, f);
     EDAB_LAUNCH("prescale");
-    monogenic_fields<T>(s, gc, plan, f, run, exp, el, work, out, batch, b0, err);
+    monogenic_fields<T>(s, gc, plan, product, f, run, exp, el, work, out, batch, b0, err);
     int32_t herr = 0;
     EDAB_CUDA(cudaMemcpyAsync(bad.data(), flag, sizeof(int32_t) * nb, cudaMemcpyDeviceToHost, s));
     EDAB_CUDA(cudaMemcpyAsync(&herr, err, sizeof herr, cudaMemcpyDeviceToHost, s));

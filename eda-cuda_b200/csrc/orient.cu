@@ -550,8 +550,8 @@ const OrientPlan& orient_plan(const Geom& g, bool f64) {
 }
 
 template <class T>
-void transform_axes(cudaStream_t s, const Geom& g, const OrientPlan& plan, const T* in, T* out, T* buf0, T* buf1,
-                    const int* kinds, const int32_t* run, int32_t* err) {
+void transform_axes(cudaStream_t s, const Geom& g, const OrientPlan& plan, TransformPrecision product, const T* in, T* out,
+                    T* buf0, T* buf1, const int* kinds, const int32_t* run, int32_t* err) {
   const int D = g.dim;
   Layout L = element_layout(g);
   const T* src = in;
@@ -561,11 +561,10 @@ void transform_axes(cudaStream_t s, const Geom& g, const OrientPlan& plan, const
     T* dst = step == D - 1 ? out : (src == buf0 ? buf1 : buf0);
     const int which = kinds[a];
     if constexpr (std::is_same_v<T, float>) {
-      const TransformPrecision mode = transform_precision();
-      if (mode == TransformPrecision::kFp32) {
+      if (product == TransformPrecision::kFp32) {
         const void* B = which == 0 ? plan.fwd[a] : (which == 1 ? plan.icos[a] : plan.isin[a]);
         rot_pass_simt<T>(s, p, g.n[a], static_cast<const T*>(B), src, dst, run);
-      } else if (mode == TransformPrecision::kBf16x3) {
+      } else if (product == TransformPrecision::kBf16x3) {
         const void* B = which == 0 ? plan.bf_fwd[a] : (which == 1 ? plan.bf_icos[a] : plan.bf_isin[a]);
         rot_pass_tc(s, p, B, true, plan.kpad[a], plan.npad[a], src, dst, run, err);
       } else {
@@ -587,10 +586,10 @@ void set_transform_precision(TransformPrecision p) {
   g_transform_precision.store(static_cast<int>(p), std::memory_order_relaxed);
 }
 
-template void transform_axes<float>(cudaStream_t, const Geom&, const OrientPlan&, const float*, float*, float*,
-                                    float*, const int*, const int32_t*, int32_t*);
-template void transform_axes<double>(cudaStream_t, const Geom&, const OrientPlan&, const double*, double*, double*,
-                                     double*, const int*, const int32_t*, int32_t*);
+template void transform_axes<float>(cudaStream_t, const Geom&, const OrientPlan&, TransformPrecision, const float*,
+                                    float*, float*, float*, const int*, const int32_t*, int32_t*);
+template void transform_axes<double>(cudaStream_t, const Geom&, const OrientPlan&, TransformPrecision, const double*,
+                                     double*, double*, double*, const int*, const int32_t*, int32_t*);
 
 int64_t orient_layout_samples(const Geom& g) {
   Layout L = element_layout(g);
@@ -669,8 +668,8 @@ void launch_riesz(cudaStream_t s, const Geom& g, int kind, int a, int b, const i
 }  // namespace
 
 template <class T>
-void orientation(cudaStream_t s, const Geom& g, const OrientPlan& plan, const T* r, Elem* el, const int32_t* run,
-                 T* const* n, T* coh, T* work, double two_sigma2, int32_t* err) {
+void orientation(cudaStream_t s, const Geom& g, const OrientPlan& plan, TransformPrecision product, const T* r, Elem* el,
+                 const int32_t* run, T* const* n, T* coh, T* work, double two_sigma2, int32_t* err) {
   const int D = g.dim;
   const int64_t F = g.batch * g.field;
   const int64_t Fw = g.batch * orient_layout_samples(g);
@@ -682,7 +681,7 @@ void orientation(cudaStream_t s, const Geom& g, const OrientPlan& plan, const T*
   auto transform = [&](const T* in, T* out, auto&& mats) {
     int kinds[kMaxDim] = {0, 0, 0};
     for (int a = 0; a < D; ++a) kinds[a] = mats(a);
-    transform_axes<T>(s, g, plan, in, out, Z, Y, kinds, run, err);
+    transform_axes<T>(s, g, plan, product, in, out, Z, Y, kinds, run, err);
   };
   // mean, then f = r - mean (the difference in double, rounded to T)
   // the means and the chunk sums at the head of Z, consumed before Z is used
@@ -820,8 +819,8 @@ int64_t monogenic_work_samples(const Geom& g) {
 }
 
 template <class T>
-void monogenic_fields(cudaStream_t s, const Geom& g, const OrientPlan& plan, const T* f, const int32_t* run,
-                      const int32_t* exp, Elem* el, T* work, T* out, int64_t out_batch, int64_t b0, int32_t* err) {
+void monogenic_fields(cudaStream_t s, const Geom& g, const OrientPlan& plan, TransformPrecision product, const T* f,
+                      const int32_t* run, const int32_t* exp, Elem* el, T* work, T* out, int64_t out_batch, int64_t b0, int32_t* err) {
   const int D = g.dim;
   const int64_t F = g.batch * g.field;
   const int64_t Fw = g.batch * orient_layout_samples(g);
@@ -849,14 +848,14 @@ void monogenic_fields(cudaStream_t s, const Geom& g, const OrientPlan& plan, con
                Y[i] = static_cast<T>(__dsub_rn(static_cast<double>(f[i]), mean[b]));
              });
   int kinds[kMaxDim] = {0, 0, 0};
-  transform_axes<T>(s, g, plan, Y, X, Z, Y, kinds, run, err);
+  transform_axes<T>(s, g, plan, product, Y, X, Z, Y, kinds, run, err);
   const dim3 grid = voxel_grid(g);
   auto component = [&](int kind, int a, int b, T* dst) {
     launch_riesz<T>(s, g, kind, a, b, run, X, Y);
     const int odd = (kind == 0 || kind == 3) ? (1 << a) : (a == b ? 0 : ((1 << a) | (1 << b)));
     int kk[kMaxDim] = {1, 1, 1};
     for (int ax = 0; ax < D; ++ax) kk[ax] = ((odd >> ax) & 1) ? 2 : 1;
-    transform_axes<T>(s, g, plan, Y, dst, Z, Y, kk, run, err);
+    transform_axes<T>(s, g, plan, product, Y, dst, Z, Y, kk, run, err);
   };
   for (int a = 0; a < D; ++a) {
     component(0, a, a, R1 + a * F);
@@ -882,14 +881,14 @@ void monogenic_fields(cudaStream_t s, const Geom& g, const OrientPlan& plan, con
   EDAB_LAUNCH("monogenic_kernel");
 }
 
-template void monogenic_fields<float>(cudaStream_t, const Geom&, const OrientPlan&, const float*, const int32_t*,
-                                      const int32_t*, Elem*, float*, float*, int64_t, int64_t, int32_t*);
-template void monogenic_fields<double>(cudaStream_t, const Geom&, const OrientPlan&, const double*, const int32_t*,
-                                       const int32_t*, Elem*, double*, double*, int64_t, int64_t, int32_t*);
+template void monogenic_fields<float>(cudaStream_t, const Geom&, const OrientPlan&, TransformPrecision, const float*,
+                                      const int32_t*, const int32_t*, Elem*, float*, float*, int64_t, int64_t, int32_t*);
+template void monogenic_fields<double>(cudaStream_t, const Geom&, const OrientPlan&, TransformPrecision, const double*,
+                                       const int32_t*, const int32_t*, Elem*, double*, double*, int64_t, int64_t, int32_t*);
 
-template void orientation<float>(cudaStream_t, const Geom&, const OrientPlan&, const float*, Elem*, const int32_t*,
-                                 float* const*, float*, float*, double, int32_t*);
-template void orientation<double>(cudaStream_t, const Geom&, const OrientPlan&, const double*, Elem*, const int32_t*,
-                                  double* const*, double*, double*, double, int32_t*);
+template void orientation<float>(cudaStream_t, const Geom&, const OrientPlan&, TransformPrecision, const float*, Elem*,
+                                 const int32_t*, float* const*, float*, float*, double, int32_t*);
+template void orientation<double>(cudaStream_t, const Geom&, const OrientPlan&, TransformPrecision, const double*, Elem*,
+                                  const int32_t*, double* const*, double*, double*, double, int32_t*);
 
 }  // namespace edab

@@ -37,8 +37,9 @@ struct OrientPlan {
   int32_t npad[kMaxDim] = {0, 0, 0};
 };
 
-// The product of the float32 transforms (process-wide; float64 always runs the FP64 product):
-// 3xTF32 and BF16x3 split products on the tensor cores, or the plain float32 SIMT product.
+// The product of the float32 transforms (float64 always runs the FP64 product): 3xTF32 and BF16x3 split
+// products on the tensor cores, or the plain float32 SIMT product. The setting is process-wide and may
+// change at any time: a call reads it once (Ctl::product) and hands it to its transforms.
 enum class TransformPrecision : int { kTf32x3 = 0, kBf16x3 = 1, kFp32 = 2 };
 TransformPrecision transform_precision();
 void set_transform_precision(TransformPrecision p);
@@ -68,15 +69,15 @@ void rot_pass_tc(cudaStream_t s, const RotPass& p, const void* basis, bool bf16,
 // (element layout) through D rotated passes, ping-ponging between buf0 and buf1 (each holding
 // every rotated layout of the batch; in may be buf1, and is then overwritten).
 template <class T>
-void transform_axes(cudaStream_t s, const Geom& g, const OrientPlan& plan, const T* in, T* out, T* buf0, T* buf1,
-                    const int* kinds, const int32_t* run, int32_t* err);
+void transform_axes(cudaStream_t s, const Geom& g, const OrientPlan& plan, TransformPrecision product, const T* in, T* out,
+                    T* buf0, T* buf1, const int* kinds, const int32_t* run, int32_t* err);
 int64_t orient_layout_samples(const Geom& g);  // the largest rotated layout of one element
 
 // n[0..D-1] and coh of every element with run[b]; el[b].w is the band's window; a non-finite
 // tensor sets el[b].nonfinite.
 template <class T>
-void orientation(cudaStream_t s, const Geom& g, const OrientPlan& plan, const T* r, Elem* el, const int32_t* run,
-                 T* const* n, T* coh, T* work, double two_sigma2, int32_t* err);
+void orientation(cudaStream_t s, const Geom& g, const OrientPlan& plan, TransformPrecision product, const T* r, Elem* el,
+                 const int32_t* run, T* const* n, T* coh, T* work, double two_sigma2, int32_t* err);
 
 // eda.monogenic of the prescaled fields f (element layout; f = x 2^-exp[b]) of the elements with
 // run[b]: the planes of out (out_batch elements; this chunk at b0): amplitude, phase, frequency
@@ -84,7 +85,7 @@ void orientation(cudaStream_t s, const Geom& g, const OrientPlan& plan, const T*
 // monogenic_work_samples(g) samples.
 int64_t monogenic_work_samples(const Geom& g);
 template <class T>
-void monogenic_fields(cudaStream_t s, const Geom& g, const OrientPlan& plan, const T* f, const int32_t* run,
-                      const int32_t* exp, Elem* el, T* work, T* out, int64_t out_batch, int64_t b0, int32_t* err);
+void monogenic_fields(cudaStream_t s, const Geom& g, const OrientPlan& plan, TransformPrecision product, const T* f,
+                      const int32_t* run, const int32_t* exp, Elem* el, T* work, T* out, int64_t out_batch, int64_t b0, int32_t* err);
 
 }  // namespace edab

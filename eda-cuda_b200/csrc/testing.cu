@@ -113,7 +113,7 @@ void run_transform(const void* x_dev, int dim, int64_t batch, const int64_t* n, 
   const OrientPlan& plan = orient_plan(g, std::is_same_v<T, double>);
   int k3[kMaxDim] = {0, 0, 0};
   for (int a = 0; a < dim; ++a) k3[a] = kinds[a];
-  transform_axes<T>(s, g, plan, in, out, b0, b1, k3, run, err);
+  transform_axes<T>(s, g, plan, transform_precision(), in, out, b0, b1, k3, run, err);
   const unsigned ob = blocks_for(batch * g.count);
   to_dense<T><<<std::min(ob, 1u << 16), kThreads, 0, s>>>(g, batch, out, static_cast<T*>(out_dev));
   EDAB_LAUNCH("to_dense");

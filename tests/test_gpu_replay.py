@@ -107,3 +107,30 @@ def test_streams_and_threads(lib):
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_the_product_of_the_transforms_changed_during_calls(lib):
+    """A call takes the product that is set when it begins, all of its transforms the same one: what calls
+    beside a thread that keeps changing it have left in the cache is what a later call issues."""
+    import eda
+
+    try:
+        for i in range(5):
+            x, ends = field((1, 60 + 8 * i, 70), np.float32, i), threading.Event()
+
+            def change():
+                while not ends.is_set():
+                    eda.set_transform_precision("bf16x3")
+                    eda.set_transform_precision("tf32x3")
+
+            t = threading.Thread(target=change)
+            t.start()
+            for _ in range(4):
+                results(x)
+            ends.set()
+            t.join()
+            for name in ("tf32x3", "bf16x3"):
+                eda.set_transform_precision(name)
+                check(lib, x)
+    finally:
+        eda.set_transform_precision("tf32x3")
