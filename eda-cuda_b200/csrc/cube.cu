@@ -104,7 +104,8 @@ void launch_pass(cudaStream_t s, const Geom& g, PassArgs<T> a) {
   const bool box = a.op == static_cast<int>(CubeOp::kBox);
   const auto bytes = box ? box_smem_bytes : ext_smem_bytes;
   int P = lines_per_cta(g, a.axis, sizeof(T), f.smem, bytes);
-  if (tune.lines > 0 && tune.lines <= 8 && bytes(n, tune.lines, rows, sizeof(T)) <= f.smem &&
+  if (tune.lines > 0 && tune.lines <= 8 && (tune.lines & (tune.lines - 1)) == 0 &&
+      bytes(n, tune.lines, rows, sizeof(T)) <= f.smem &&
       (!rows || tune.lines <= std::max<int64_t>(1, g.rows))) {
     P = tune.lines;
   }

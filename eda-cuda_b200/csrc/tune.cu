@@ -56,6 +56,9 @@ TuneKey key_of(const Geom& g, size_t es) {
   return TuneKey{static_cast<int>(es), g.dim, g.n[0], g.n[1], g.n[2], bucket_of(g.batch)};
 }
 
+// The lines per CTA that the passes are built for; 0: the default.
+bool valid_lines(int32_t lines) { return lines == 0 || lines == 1 || lines == 2 || lines == 4 || lines == 8; }
+
 void load_file_locked(const std::string& path) {
   std::ifstream in(path);
   if (!in) throw std::invalid_argument("eda: cannot read the tuning cache " + path);
@@ -69,7 +72,7 @@ void load_file_locked(const std::string& path) {
           r.tune.seq_share >> r.us_default >> r.us_best)) {
       throw std::invalid_argument("eda: malformed tuning cache line: " + line);
     }
-    if ((k.es != 4 && k.es != 8) || k.dim < 1 || k.dim > kMaxDim || r.tune.lines < 0 || r.tune.lines > 8 ||
+    if ((k.es != 4 && k.es != 8) || k.dim < 1 || k.dim > kMaxDim || !valid_lines(r.tune.lines) ||
         r.tune.groups < 0 || r.tune.groups > 4 || r.tune.seq_share < 0 || r.tune.seq_share > 64) {
       throw std::invalid_argument("eda: out-of-range tuning cache line: " + line);
     }

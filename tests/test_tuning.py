@@ -44,6 +44,19 @@ def test_bad_lines_are_rejected(core, tmp_path, line):
         core.tuning_load(str(p))
 
 
+@pytest.mark.parametrize("lines", range(-1, 18))
+def test_lines_that_the_passes_are_not_built_for_are_rejected(core, tmp_path, lines):
+    p = tmp_path / "lines.txt"
+    p.write_text(f"4 2 512 512 1 6 {lines} 2 8 1 1\n")
+    if lines in (0, 1, 2, 4, 8):
+        core.tuning_load(str(p))
+        assert [ln.split()[6] for ln in core.tuning_dump().splitlines() if not ln.startswith("#")] == [str(lines)]
+    else:
+        with pytest.raises(ValueError):
+            core.tuning_load(str(p))
+        assert [ln for ln in core.tuning_dump().splitlines() if not ln.startswith("#")] == []
+
+
 def test_missing_file_is_rejected(core, tmp_path):
     with pytest.raises(ValueError):
         core.tuning_load(str(tmp_path / "absent.txt"))
