@@ -392,13 +392,12 @@ void box_allow_smem(int bytes) {
 
 template <class T>
 void launch_box(cudaStream_t s, const Geom& g, const PassArgs<T>& a, int P, bool rows, dim3 grid, size_t smem) {
-  if (rows && P == 8) box_pass<T, 8, true><<<grid, kCubeThreads, smem, s>>>(g, a);
-  else if (rows) box_pass<T, 1, true><<<grid, kCubeThreads, smem, s>>>(g, a);
-  else if (P == 1) box_pass<T, 1, false><<<grid, kCubeThreads, smem, s>>>(g, a);
-  else if (P == 2) box_pass<T, 2, false><<<grid, kCubeThreads, smem, s>>>(g, a);
-  else if (P == 4) box_pass<T, 4, false><<<grid, kCubeThreads, smem, s>>>(g, a);
-  else box_pass<T, 8, false><<<grid, kCubeThreads, smem, s>>>(g, a);
-  EDAB_LAUNCH("box_pass");
+  if (rows && P == 8) enqueue(box_pass<T, 8, true>, grid, kCubeThreads, smem, s, g, a);
+  else if (rows) enqueue(box_pass<T, 1, true>, grid, kCubeThreads, smem, s, g, a);
+  else if (P == 1) enqueue(box_pass<T, 1, false>, grid, kCubeThreads, smem, s, g, a);
+  else if (P == 2) enqueue(box_pass<T, 2, false>, grid, kCubeThreads, smem, s, g, a);
+  else if (P == 4) enqueue(box_pass<T, 4, false>, grid, kCubeThreads, smem, s, g, a);
+  else enqueue(box_pass<T, 8, false>, grid, kCubeThreads, smem, s, g, a);
 }
 
 template void box_allow_smem<float>(int);

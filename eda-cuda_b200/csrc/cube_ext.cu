@@ -450,13 +450,12 @@ void ext_allow_smem(int bytes) {
 template <class T>
 void launch_ext(cudaStream_t s, const Geom& g, const PassArgs<T>& a, int P, bool rows, dim3 grid, size_t smem) {
   if (rows && P != 8 && a.zr == 1 && a.zf == 1) smem -= static_cast<size_t>(group_elems<T>(geom_n(g, a.axis), P, rows)) * sizeof(T);
-  if (rows && P == 8) ext_pass<T, 8, true><<<grid, kCubeThreads, smem, s>>>(g, a);
-  else if (rows) ext_pass<T, 1, true><<<grid, kCubeThreads, smem, s>>>(g, a);
-  else if (P == 1) ext_pass<T, 1, false><<<grid, kCubeThreads, smem, s>>>(g, a);
-  else if (P == 2) ext_pass<T, 2, false><<<grid, kCubeThreads, smem, s>>>(g, a);
-  else if (P == 4) ext_pass<T, 4, false><<<grid, kCubeThreads, smem, s>>>(g, a);
-  else ext_pass<T, 8, false><<<grid, kCubeThreads, smem, s>>>(g, a);
-  EDAB_LAUNCH("ext_pass");
+  if (rows && P == 8) enqueue(ext_pass<T, 8, true>, grid, kCubeThreads, smem, s, g, a);
+  else if (rows) enqueue(ext_pass<T, 1, true>, grid, kCubeThreads, smem, s, g, a);
+  else if (P == 1) enqueue(ext_pass<T, 1, false>, grid, kCubeThreads, smem, s, g, a);
+  else if (P == 2) enqueue(ext_pass<T, 2, false>, grid, kCubeThreads, smem, s, g, a);
+  else if (P == 4) enqueue(ext_pass<T, 4, false>, grid, kCubeThreads, smem, s, g, a);
+  else enqueue(ext_pass<T, 8, false>, grid, kCubeThreads, smem, s, g, a);
 }
 
 template void ext_allow_smem<float>(int);

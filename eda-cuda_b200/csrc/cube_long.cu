@@ -533,10 +533,9 @@ void launch_long(cudaStream_t s, const Geom& g, const PassArgs<T>& a, void* line
   const T* out_end = a.out0 + (a.rungs - 1) * a.out_stride + g.batch * g.field;
   if (box && !a.bits && (a.in0 >= out_end || a.in0 + g.batch * g.field <= a.out0)) {
     L.line = const_cast<T*>(a.in0);
-    EDAB_CUDA(cudaMemsetAsync(L.done, 0, static_cast<size_t>(a.rungs) * B * sizeof(int32_t), s));
+    enqueue_zero(L.done, static_cast<size_t>(a.rungs) * B * sizeof(int32_t), s);
   } else {
-    long_input<T><<<dim3(in_x, B), kThreads, 0, s>>>(g, a, L, box ? a.rungs * static_cast<int32_t>(g.batch) : 0);
-    EDAB_LAUNCH("long_input");
+    enqueue(long_input<T>, dim3(in_x, B), kThreads, 0, s, g, a, L, box ? a.rungs * static_cast<int32_t>(g.batch) : 0);
   }
   const int32_t tile = long_tile(g, static_cast<int64_t>(a.rungs) * nf, sms);
   const unsigned tiles = static_cast<unsigned>((g.n_last + tile - 1) / tile);
@@ -546,8 +545,7 @@ void launch_long(cudaStream_t s, const Geom& g, const PassArgs<T>& a, void* line
     once_on_device(reinterpret_cast<const void*>(long_ext<T>), [&] {
       EDAB_CUDA(cudaFuncSetAttribute(long_ext<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_cap)));
     });
-    long_ext<T><<<dim3(tiles, B, static_cast<unsigned>(a.rungs * nf)), kThreads, smem, s>>>(g, a, L, tile);
-    EDAB_LAUNCH("long_ext");
+    enqueue(long_ext<T>, dim3(tiles, B, static_cast<unsigned>(a.rungs * nf)), kThreads, smem, s, g, a, L, tile);
     return;
   }
   const size_t carries = static_cast<size_t>(2) * L.TSL * sizeof(T);
@@ -558,10 +556,8 @@ void launch_long(cudaStream_t s, const Geom& g, const PassArgs<T>& a, void* line
     EDAB_CUDA(cudaFuncSetAttribute(long_box<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_cap)));
   });
   const unsigned tx = static_cast<unsigned>(std::clamp<int64_t>((2 * L.TSL / 4 + kThreads - 1) / kThreads, 1, 16));
-  long_totals<T><<<dim3(tx, B, static_cast<unsigned>(a.rungs)), kThreads, carries, s>>>(g, a, L, tile);
-  EDAB_LAUNCH("long_totals");
-  long_box<T><<<dim3(tiles, B, static_cast<unsigned>(a.rungs)), kThreads, smem, s>>>(g, a, L, tile);
-  EDAB_LAUNCH("long_box");
+  enqueue(long_totals<T>, dim3(tx, B, static_cast<unsigned>(a.rungs)), kThreads, carries, s, g, a, L, tile);
+  enqueue(long_box<T>, dim3(tiles, B, static_cast<unsigned>(a.rungs)), kThreads, smem, s, g, a, L, tile);
 }
 
 template void launch_long<float>(cudaStream_t, const Geom&, const PassArgs<float>&, void*, void*, int, size_t);

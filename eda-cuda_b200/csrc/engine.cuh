@@ -9,6 +9,8 @@
 // reductions or exact order statistics.
 #pragma once
 
+#include "launch.hpp"
+
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -42,8 +44,8 @@ void cuda_fail(cudaError_t e, const char* what, const char* file, int line);
     const cudaError_t e_ = (call);                                        \
     if (e_ != cudaSuccess) ::edab::cuda_fail(e_, #call, __FILE__, __LINE__); \
   } while (0)
-// Every kernel launch of the engine is followed by EDAB_LAUNCH: it checks the launch and counts it
-// for the instrumentation (profile.cu).
+// Every kernel launch is counted for the instrumentation (profile.cu) and checked: by enqueue (launch.hpp:
+// the engine's steps), or by EDAB_LAUNCH after it.
 void note_launch();
 // Runs set(), which sets attributes of kernel `key` on the current device (such as its dynamic
 // shared-memory limit: they are per device), on the first call for that kernel and device. Every
@@ -345,8 +347,7 @@ __global__ void __launch_bounds__(kThreads) voxel_kernel(Geom g, Run run, F f) {
 }
 template <class Run, class F>
 void for_voxels(cudaStream_t s, const Geom& g, Run run, F f) {
-  voxel_kernel<<<voxel_grid(g), kThreads, 0, s>>>(g, run, f);
-  EDAB_LAUNCH("voxel_kernel");
+  enqueue(voxel_kernel<Run, F>, voxel_grid(g), kThreads, 0, s, g, run, f);
 }
 // Every padded sample (pads included).
 template <class F>
@@ -360,8 +361,7 @@ template <class F>
 void for_samples(cudaStream_t s, int64_t total, F f) {
   int64_t blocks = (total + kThreads * 4 - 1) / (kThreads * 4);
   blocks = blocks < 1 ? 1 : (blocks > (1 << 20) ? (1 << 20) : blocks);
-  sample_kernel<<<static_cast<unsigned>(blocks), kThreads, 0, s>>>(total, f);
-  EDAB_LAUNCH("sample_kernel");
+  enqueue(sample_kernel<F>, static_cast<unsigned>(blocks), kThreads, 0, s, total, f);
 }
 template <class F>
 __global__ void element_kernel(int64_t B, F f) {
@@ -370,8 +370,7 @@ __global__ void element_kernel(int64_t B, F f) {
 }
 template <class F>
 void for_elements(cudaStream_t s, int64_t B, F f) {
-  element_kernel<<<blocks_for(B), kThreads, 0, s>>>(B, f);
-  EDAB_LAUNCH("element_kernel");
+  enqueue(element_kernel<F>, blocks_for(B), kThreads, 0, s, B, f);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -685,15 +685,7 @@ class Engine {
     put(c_.tau);
     put(base_);
     put(L_);
-    replays_->run(key, s_, [&](cudaStream_t s) {
-      struct Stream {  // the engine's stream again, also after an error
-        cudaStream_t& at;
-        cudaStream_t kept;
-        ~Stream() { at = kept; }
-      } back{s_, s_};
-      s_ = s;
-      body();
-    });
+    replays_->run(key, s_, body);
   }
   void noise(const T* r, unsigned axes, const int32_t* run, double* out);
   void noise_per_axis(const T* r, const int32_t* run, double* out);
@@ -1118,11 +1110,10 @@ void Engine<T>::orientation_and_build() {
   }
   const dim3 grid = voxel_grid(g_);
   switch (g_.dim) {
-    case 1: element_extent<T, 1><<<grid, kThreads, 0, s_>>>(g_, c_, L_, coh_, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, t_, lo_, el_, on); break;
-    case 2: element_extent<T, 2><<<grid, kThreads, 0, s_>>>(g_, c_, L_, coh_, n_[0], n_[1], nullptr, o_[0], o_[1], nullptr, t_, lo_, el_, on); break;
-    default: element_extent<T, 3><<<grid, kThreads, 0, s_>>>(g_, c_, L_, coh_, n_[0], n_[1], n_[2], o_[0], o_[1], o_[2], t_, lo_, el_, on); break;
+    case 1: enqueue(element_extent<T, 1>, grid, kThreads, 0, s_, g_, c_, L_, coh_, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, t_, lo_, el_, on); break;
+    case 2: enqueue(element_extent<T, 2>, grid, kThreads, 0, s_, g_, c_, L_, coh_, n_[0], n_[1], nullptr, o_[0], o_[1], nullptr, t_, lo_, el_, on); break;
+    default: enqueue(element_extent<T, 3>, grid, kThreads, 0, s_, g_, c_, L_, coh_, n_[0], n_[1], n_[2], o_[0], o_[1], o_[2], t_, lo_, el_, on); break;
   }
-  EDAB_LAUNCH("element_extent");
 }
 
 // return_orientation: n with the canonical sign (the first component of magnitude above the dtype's
@@ -1194,8 +1185,7 @@ void Engine<T>::weights(int32_t nrm) {
     const int j = static_cast<int>(i % kMaxRungs);
     if (on[b] && j < el[b].n_rungs) el[b].rung_lw[j] = log(static_cast<double>(el[b].rung_w[j]));
   });
-  element_rungs<T><<<voxel_grid(g_), kThreads, 0, s_>>>(g_, lo_, t_, el_, on);
-  EDAB_LAUNCH("element_rungs");
+  enqueue(element_rungs<T>, voxel_grid(g_), kThreads, 0, s_, g_, lo_, t_, el_, on);
   int32_t* rw = rung_win_;
   const int64_t B = B_;
   for_samples(s_, B_ * kMaxRungs, [=] __device__(int64_t i) {
@@ -1228,7 +1218,7 @@ void Engine<T>::op(int which, const T* in, const GatherOut<T>& out, int32_t nrm)
   const T* o1 = o_[1];
   const T* o2 = o_[2];
 #define EDAB_GATHER(D, OP) \
-  gather_kernel<T, D, OP><<<grid, kThreads, 0, s_>>>(g_, el_, on, lo_, t_, o0, o1, o2, rung0_, rung1_, out)
+  enqueue(gather_kernel<T, D, OP>, grid, kThreads, 0, s_, g_, el_, on, lo_, t_, o0, o1, o2, rung0_, rung1_, out)
   if (g_.dim == 1) {
     if (which == 0) EDAB_GATHER(1, 0); else if (which == 2) EDAB_GATHER(1, 2); else EDAB_GATHER(1, 3);
   } else if (g_.dim == 2) {
@@ -1237,7 +1227,6 @@ void Engine<T>::op(int which, const T* in, const GatherOut<T>& out, int32_t nrm)
     if (which == 0) EDAB_GATHER(3, 0); else if (which == 2) EDAB_GATHER(3, 2); else EDAB_GATHER(3, 3);
   }
 #undef EDAB_GATHER
-  EDAB_LAUNCH("gather_kernel");
 }
 
 // The mean envelope of h: the extremes with what `ext` stores of them (the middle always), then the box
@@ -1369,8 +1358,7 @@ void Engine<T>::sifts(int32_t nrm) {
     }
     const dim3 grid = voxel_grid(g_);
     const SiftBlend<T> blend{gk_, e_, up_, lo_f_, plain_, Mn_};
-    sift_step_kernel<T><<<grid, kThreads, 0, s_>>>(g_, el_, r_, h_, blend, a_, hn_);
-    EDAB_LAUNCH("sift_step_kernel");
+    enqueue(sift_step_kernel<T>, grid, kThreads, 0, s_, g_, el_, r_, h_, blend, a_, hn_);
     {
       T* hh = h_;
       const T* hn = hn_;

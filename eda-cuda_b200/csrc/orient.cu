@@ -187,8 +187,7 @@ void rot_pass_simt(cudaStream_t s, const RotPass& p, int32_t n, const T* M, cons
   const int64_t batch = p.M / p.rows;
   const dim3 grid(static_cast<unsigned>((d.N + kBN - 1) / kBN), static_cast<unsigned>((d.M + kBM - 1) / kBM),
                   static_cast<unsigned>(batch * outer));
-  gemm_simt<T><<<grid, kSimtThreads, 0, s>>>(d, in, M, out, run);
-  EDAB_LAUNCH("gemm_simt");
+  enqueue(gemm_simt<T>, grid, kSimtThreads, 0, s, d, in, M, out, run);
 }
 
 // The element's mean in double, deterministic for a shape: fixed chunks of kMeanChunk padded
@@ -658,11 +657,10 @@ void launch_riesz(cudaStream_t s, const Geom& g, int kind, int a, int b, const i
   dim3 grid = voxel_grid(g, 1);
   grid.y = static_cast<unsigned>(std::clamp<int64_t>((g.batch + kRieszPer - 1) / kRieszPer, 1, 65535));
   switch (g.dim) {
-    case 1: riesz_spectrum<T, 1><<<grid, 256, 0, s>>>(g, kind, a, b, run, X, Y); break;
-    case 2: riesz_spectrum<T, 2><<<grid, 256, 0, s>>>(g, kind, a, b, run, X, Y); break;
-    default: riesz_spectrum<T, 3><<<grid, 256, 0, s>>>(g, kind, a, b, run, X, Y); break;
+    case 1: enqueue(riesz_spectrum<T, 1>, grid, 256, 0, s, g, kind, a, b, run, X, Y); break;
+    case 2: enqueue(riesz_spectrum<T, 2>, grid, 256, 0, s, g, kind, a, b, run, X, Y); break;
+    default: enqueue(riesz_spectrum<T, 3>, grid, 256, 0, s, g, kind, a, b, run, X, Y); break;
   }
-  EDAB_LAUNCH("riesz_spectrum");
 }
 
 }  // namespace
@@ -688,11 +686,9 @@ void orientation(cudaStream_t s, const Geom& g, const OrientPlan& plan, Transfor
   const int64_t nchunks = (g.field + kMeanChunk - 1) / kMeanChunk;
   double* mean = reinterpret_cast<double*>(Z);
   double* part = mean + g.batch;
-  mean_partial<T><<<dim3(static_cast<unsigned>(nchunks), static_cast<unsigned>(g.batch)), 256, 0, s>>>(g, r, run, part,
+  enqueue(mean_partial<T>, dim3(static_cast<unsigned>(nchunks), static_cast<unsigned>(g.batch)), 256, 0, s, g, r, run, part,
                                                                                                        nchunks);
-  EDAB_LAUNCH("mean_partial");
-  mean_final<<<blocks_for(g.batch), 256, 0, s>>>(g.batch, g.count, run, part, nchunks, mean);
-  EDAB_LAUNCH("mean_final");
+  enqueue(mean_final, blocks_for(g.batch), 256, 0, s, g.batch, g.count, run, part, nchunks, mean);
   for_voxels(s, g, [=] __device__(int64_t b) { return run[b] != 0; },
              [=] __device__(int64_t b, int64_t, int64_t i) {
                Y[i] = static_cast<T>(__dsub_rn(static_cast<double>(r[i]), mean[b]));
@@ -730,9 +726,8 @@ void orientation(cudaStream_t s, const Geom& g, const OrientPlan& plan, Transfor
     }
   }
   const dim3 grid = voxel_grid(g);
-  if (D == 2) tensor_eigen<T, 2><<<grid, 256, 0, s>>>(g, run, R1, R2, n[0], n[1], nullptr, coh, el);
-  else tensor_eigen<T, 3><<<grid, 256, 0, s>>>(g, run, R1, R2, n[0], n[1], n[2], coh, el);
-  EDAB_LAUNCH("tensor_eigen");
+  if (D == 2) enqueue(tensor_eigen<T, 2>, grid, 256, 0, s, g, run, R1, R2, n[0], n[1], nullptr, coh, el);
+  else enqueue(tensor_eigen<T, 3>, grid, 256, 0, s, g, run, R1, R2, n[0], n[1], n[2], coh, el);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -838,11 +833,9 @@ void monogenic_fields(cudaStream_t s, const Geom& g, const OrientPlan& plan, Tra
   const int64_t nchunks = (g.field + kMeanChunk - 1) / kMeanChunk;
   double* mean = reinterpret_cast<double*>(Z);
   double* part = mean + g.batch;
-  mean_partial<T><<<dim3(static_cast<unsigned>(nchunks), static_cast<unsigned>(g.batch)), 256, 0, s>>>(g, f, run, part,
+  enqueue(mean_partial<T>, dim3(static_cast<unsigned>(nchunks), static_cast<unsigned>(g.batch)), 256, 0, s, g, f, run, part,
                                                                                                        nchunks);
-  EDAB_LAUNCH("mean_partial");
-  mean_final<<<blocks_for(g.batch), 256, 0, s>>>(g.batch, g.count, run, part, nchunks, mean);
-  EDAB_LAUNCH("mean_final");
+  enqueue(mean_final, blocks_for(g.batch), 256, 0, s, g.batch, g.count, run, part, nchunks, mean);
   for_voxels(s, g, [=] __device__(int64_t b) { return run[b] != 0; },
              [=] __device__(int64_t b, int64_t, int64_t i) {
                Y[i] = static_cast<T>(__dsub_rn(static_cast<double>(f[i]), mean[b]));
@@ -868,17 +861,16 @@ void monogenic_fields(cudaStream_t s, const Geom& g, const OrientPlan& plan, Tra
       component(4, a, b, DR + p * F);
     }
   }
-  if (D == 2) tensor_eigen<T, 2><<<grid, 256, 0, s>>>(g, run, R1, R2, N, N + F, nullptr, C, el);
-  else if (D == 3) tensor_eigen<T, 3><<<grid, 256, 0, s>>>(g, run, R1, R2, N, N + F, N + 2 * F, C, el);
+  if (D == 2) enqueue(tensor_eigen<T, 2>, grid, 256, 0, s, g, run, R1, R2, N, N + F, nullptr, C, el);
+  else if (D == 3) enqueue(tensor_eigen<T, 3>, grid, 256, 0, s, g, run, R1, R2, N, N + F, N + 2 * F, C, el);
   if (D >= 2) EDAB_LAUNCH("tensor_eigen");
   const double tiny = std::is_same_v<T, float> ? 1.17549435082228750797e-38 : 1e-300;
   const T zero = static_cast<T>(std::is_same_v<T, float> ? std::ldexp(1.0, -14) : std::ldexp(1.0, -30));
   switch (D) {
-    case 1: monogenic_kernel<T, 1><<<grid, 256, 0, s>>>(g, f, R1, DF, DR, N, C, exp, tiny, zero, out, out_batch, b0); break;
-    case 2: monogenic_kernel<T, 2><<<grid, 256, 0, s>>>(g, f, R1, DF, DR, N, C, exp, tiny, zero, out, out_batch, b0); break;
-    default: monogenic_kernel<T, 3><<<grid, 256, 0, s>>>(g, f, R1, DF, DR, N, C, exp, tiny, zero, out, out_batch, b0); break;
+    case 1: enqueue(monogenic_kernel<T, 1>, grid, 256, 0, s, g, f, R1, DF, DR, N, C, exp, tiny, zero, out, out_batch, b0); break;
+    case 2: enqueue(monogenic_kernel<T, 2>, grid, 256, 0, s, g, f, R1, DF, DR, N, C, exp, tiny, zero, out, out_batch, b0); break;
+    default: enqueue(monogenic_kernel<T, 3>, grid, 256, 0, s, g, f, R1, DF, DR, N, C, exp, tiny, zero, out, out_batch, b0); break;
   }
-  EDAB_LAUNCH("monogenic_kernel");
 }
 
 template void monogenic_fields<float>(cudaStream_t, const Geom&, const OrientPlan&, TransformPrecision, const float*,

@@ -474,8 +474,7 @@ void launch(cudaStream_t s, const RotPass& p, const void* basis, int32_t kpad, i
     EDAB_CUDA(cudaFuncSetAttribute(gemm_tc<BF16, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmem));
   });
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(ro.tiles, sms));
-  gemm_tc<BF16, BN><<<grid, kThreadsTc, L::kSmem, s>>>(ta, tb, ro, out, run, err);
-  EDAB_LAUNCH("gemm_tc");
+  enqueue(gemm_tc<BF16, BN>, grid, kThreadsTc, L::kSmem, s, ta, tb, ro, out, run, err);
 }
 
 }  // namespace tc

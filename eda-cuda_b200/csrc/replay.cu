@@ -11,11 +11,9 @@ void Replays::clear() {
     if (e.exec) cudaGraphExecDestroy(e.exec);
   }
   entries_.clear();
-  if (capture_) cudaStreamDestroy(capture_);
-  capture_ = nullptr;
 }
 
-void Replays::run(const std::string& key, cudaStream_t s, const std::function<void(cudaStream_t)>& issue) {
+void Replays::run(const std::string& key, cudaStream_t s, const std::function<void()>& issue) {
   auto it = entries_.find(key);
   if (it == entries_.end()) {
     if (entries_.size() >= kMost) {
@@ -30,34 +28,26 @@ void Replays::run(const std::string& key, cudaStream_t s, const std::function<vo
       entries_.erase(old);
     }
     entries_[key].used = ++clock_;
-    issue(s);
+    issue();
     return;
   }
   Entry& e = it->second;
   e.used = ++clock_;
   if (!e.exec && !e.refused) {
-    if (!capture_) EDAB_CUDA(cudaStreamCreateWithFlags(&capture_, cudaStreamNonBlocking));
-    cudaGraph_t graph = nullptr;
-    bool issued = false;
-    EDAB_CUDA(cudaStreamBeginCapture(capture_, cudaStreamCaptureModeRelaxed));
     try {
-      issue(capture_);
-      issued = true;
+      Sequence q;
+      issue();
+      e.exec = q.instantiate();
     } catch (const std::exception&) {
-      // the capture ends below; the sequence is issued directly, where an error that is its own shows
+      // the sequence is issued directly, where an error that is its own shows
     }
-    const cudaError_t ended = cudaStreamEndCapture(capture_, &graph);
-    if (issued && ended == cudaSuccess && graph) {
-      if (cudaGraphInstantiate(&e.exec, graph, 0) != cudaSuccess) e.exec = nullptr;
-    }
-    if (graph) cudaGraphDestroy(graph);
     if (!e.exec) {
       e.refused = true;
       (void)cudaGetLastError();
     }
   }
   if (e.exec) EDAB_CUDA(cudaGraphLaunch(e.exec, s));
-  else issue(s);
+  else issue();
 }
 
 }  // namespace edab

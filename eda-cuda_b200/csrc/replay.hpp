@@ -3,8 +3,8 @@
 // issues a fixed sequence of launches: it depends on the geometry, the call's constants, the
 // workspace's address and a count or two (the rungs), never on the data. For small fields the
 // sequence is bound by its launches (one signal of 2048 samples: 533 launches, 2.5 ms of kernels in
-// 4.8 ms), so a sequence that a thread's workspace runs for the second time is captured, and from
-// then on launched as one graph.
+// 4.8 ms), so a sequence that a thread's workspace runs for the second time is built as a graph (launch.hpp),
+// and from then on launched as one.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -19,22 +19,21 @@ namespace edab {
 class Replays {
  public:
   ~Replays() { clear(); }
-  // Runs `issue`, which enqueues the sequence of `key` on the stream that it is given, on stream s:
-  // directly the first time that the key is seen, as its graph afterwards.
-  void run(const std::string& key, cudaStream_t s, const std::function<void(cudaStream_t)>& issue);
+  // Runs `issue`, which enqueues the sequence of `key`, on stream s: directly the first time that the key is
+  // seen, as its graph afterwards.
+  void run(const std::string& key, cudaStream_t s, const std::function<void()>& issue);
   void clear();  // the graphs hold addresses of the workspace: none outlives its buffer
 
  private:
   struct Entry {
     cudaGraphExec_t exec = nullptr;
-    bool refused = false;  // could not be captured: always issued directly
+    bool refused = false;  // could not be built: always issued directly
     uint64_t used = 0;
   };
   // The least recently used sequence leaves beyond this many: a program that cycles through more never
-  // comes to its second use, so it pays for no capture.
+  // comes to its second use, so it builds no graph.
   static constexpr size_t kMost = 64;
   std::map<std::string, Entry> entries_;
-  cudaStream_t capture_ = nullptr;  // (the legacy stream cannot be captured)
   uint64_t clock_ = 0;
 };
 

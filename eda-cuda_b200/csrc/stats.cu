@@ -1220,11 +1220,9 @@ void field_totals(cudaStream_t s, const Geom& g, const T* f, double* energy, dou
   if (g.n_last > kMaxSteps * 1024) throw std::invalid_argument("edab: a row is too long for the energy sums");
   const bool per_row = g.n_last > 1024;
   const int64_t blocks = std::clamp<int64_t>(per_row ? total : (total + (kRowThreads<T> / 32) - 1) / (kRowThreads<T> / 32), 1, int64_t{1} << 20);
-  row_partials<T><<<static_cast<unsigned>(blocks), kRowThreads<T>, 0, s>>>(f, g, rows, nonfinite, per_row);
-  EDAB_LAUNCH("row_partials");
+  enqueue(row_partials<T>, static_cast<unsigned>(blocks), kRowThreads<T>, 0, s, f, g, rows, nonfinite, per_row);
   const unsigned eb = static_cast<unsigned>(std::clamp<int64_t>(g.batch, 1, 65535));
-  element_totals<<<eb, kThreads, 0, s>>>(g, rows, energy, amax);
-  EDAB_LAUNCH("element_totals");
+  enqueue(element_totals, eb, kThreads, 0, s, g, rows, energy, amax);
 }
 
 constexpr int64_t kMaskKeys = 32;
@@ -1270,7 +1268,7 @@ void select_grid(cudaStream_t s, const Geom& g, const SelView<T>& a, double q, c
   const SelCand<K> cand = (sizeof(K) == 8 || EDAB_SEL_CAND32) ? cand_of<K>(g, scratch) : SelCand<K>{};
   const size_t clear = static_cast<size_t>(reinterpret_cast<char*>(cand_of<K>(g, scratch).n) - static_cast<char*>(scratch)) +
                        static_cast<size_t>(g.batch) * sizeof(unsigned long long);
-  EDAB_CUDA(cudaMemsetAsync(scratch, 0, clear, s));
+  enqueue_zero(scratch, clear, s);
   // CTAs per element: 64 items per thread, and for small batches enough CTAs for 8 per SM (at
   // least 4 items per thread)
   const int64_t by_items = (a.items + int64_t{kThreads} * 64 - 1) / (int64_t{kThreads} * 64);
@@ -1278,9 +1276,8 @@ void select_grid(cudaStream_t s, const Geom& g, const SelView<T>& a, double q, c
                                          std::max<int64_t>(1, a.items / (int64_t{kThreads} * 4)));
   const unsigned ctas = static_cast<unsigned>(std::clamp<int64_t>(std::max(by_items, fill), 1, 1024));
   for (int pass = 0; pass < kDigits; ++pass) {
-    select_grid_count<T, K><<<dim3(ctas, static_cast<unsigned>(g.batch)), kThreads, 0, s>>>(g, a, run, st, table, pass,
+    enqueue(select_grid_count<T, K>, dim3(ctas, static_cast<unsigned>(g.batch)), kThreads, 0, s, g, a, run, st, table, pass,
                                                                                           cand, q, out, count);
-    EDAB_LAUNCH("select_grid_count");
   }
 }
 
@@ -1292,15 +1289,12 @@ const int32_t* select_split(cudaStream_t s, const Geom& g, const SelView<T>& a, 
   auto* st = static_cast<SplitState<K>*>(scratch);
   int32_t* mask = split_mask(g, cand);
   const unsigned B = static_cast<unsigned>(g.batch);
-  split_pivots<T, K><<<B, kSplitThreads, 0, s>>>(g, a, run, q, st);
-  EDAB_LAUNCH("split_pivots");
+  enqueue(split_pivots<T, K>, B, kSplitThreads, 0, s, g, a, run, q, st);
   // 8 CTAs per SM in all, at least 16 items per thread
   const int64_t fill = (int64_t{8} * sms + g.batch - 1) / g.batch;
   const unsigned ctas = static_cast<unsigned>(std::clamp<int64_t>(fill, 1, std::max<int64_t>(1, a.items / (int64_t{kThreads} * 16))));
-  split_count<T, K><<<dim3(ctas, B), kThreads, 0, s>>>(g, a, run, st, cand);
-  EDAB_LAUNCH("split_count");
-  split_finish<K><<<B, kSplitThreads, 0, s>>>(run, st, cand, q, out, count, mask);
-  EDAB_LAUNCH("split_finish");
+  enqueue(split_count<T, K>, dim3(ctas, B), kThreads, 0, s, g, a, run, st, cand);
+  enqueue(split_finish<K>, B, kSplitThreads, 0, s, run, st, cand, q, out, count, mask);
   return mask;
 }
 
@@ -1351,8 +1345,7 @@ void select(cudaStream_t s, const Geom& g, const Sel<T>& sel, double q, const in
       once_on_device(reinterpret_cast<const void*>(kernel), [&] {
         EDAB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmallBytes)));
       });
-      kernel<<<static_cast<unsigned>(g.batch), th, small, s>>>(g, a, run, q, out, count);
-      EDAB_LAUNCH("select_small");
+      enqueue(kernel, static_cast<unsigned>(g.batch), th, small, s, g, a, run, q, out, count);
     };
     if constexpr (std::is_same_v<T, float>) {
       if (narrow) {
@@ -1378,24 +1371,12 @@ void select(cudaStream_t s, const Geom& g, const Sel<T>& sel, double q, const in
   // CTAs per element: about 16 items per thread (4 in a small batch), up to a cluster of 8
   const int64_t per_cta = many ? int64_t{kThreads} * 16 : int64_t{kSelWide} * 4;
   const unsigned ctas = static_cast<unsigned>(std::clamp<int64_t>((a.items + per_cta - 1) / per_cta, 1, kSelClusterMax));
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(ctas, static_cast<unsigned>(g.batch));
-  cfg.blockDim = dim3(many ? kThreads : kSelWide);
-  cfg.dynamicSmemBytes = kSelSmem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = ctas;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   const auto launch = [&](auto kernel, auto cand) {
     once_on_device(reinterpret_cast<const void*>(kernel), [&] {
       EDAB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSelSmem)));
     });
-    EDAB_CUDA(cudaLaunchKernelEx(&cfg, kernel, g, a, run, q, out, count, cand));
-    EDAB_LAUNCH("select_cluster");
+    enqueue_clusters(ctas, kernel, dim3(ctas, static_cast<unsigned>(g.batch)), many ? kThreads : kSelWide, kSelSmem, s, g, a, run,
+                     q, out, count, cand);
   };
   if constexpr (std::is_same_v<T, float>) {
     if (sel.center == nullptr) {
@@ -1911,14 +1892,12 @@ void sig_flags(cudaStream_t s, const Geom& g, const T* r, const T* tau, uint8_t*
         EDAB_CUDA(cudaFuncSetAttribute(flags_long<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(cap)));
       });
       const int64_t fill = std::clamp<int64_t>((8 * static_cast<int64_t>(sms) + g.batch - 1) / g.batch, 1, 16);
-      flags_long<T><<<dim3(static_cast<unsigned>(fill), static_cast<unsigned>(g.batch)), kThreads, ext_bytes, s>>>(
+      enqueue(flags_long<T>, dim3(static_cast<unsigned>(fill), static_cast<unsigned>(g.batch)), kThreads, ext_bytes, s, 
           g, r, tau, flags, el, run);
-      EDAB_LAUNCH("flags_long");
       continue;
     }
-    flags_pass<T><<<dim3(static_cast<unsigned>(groups_of(P) * parts), static_cast<unsigned>(g.batch)), kThreads, bytes(P), s>>>(
+    enqueue(flags_pass<T>, dim3(static_cast<unsigned>(groups_of(P) * parts), static_cast<unsigned>(g.batch)), kThreads, bytes(P), s, 
         g, a, r, tau, flags, el, run, P, LX, parts);
-    EDAB_LAUNCH("flags_pass");
   }
 }
 
@@ -1929,9 +1908,8 @@ void ccl(cudaStream_t s, const Geom& g, const uint8_t* mask, uint8_t bits, int32
   const int64_t col_tiles = (g.pitch + tile_cols - 1) / tile_cols;
   const int64_t tiles = (g.rows + tile_rows - 1) / tile_rows * col_tiles;
   if (tiles > 0x7fffffffLL || g.batch > 65535) throw std::invalid_argument("edab: components: grid too large");
-  ccl_tiles<<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(g.batch)), kThreads, 0, s>>>(
+  enqueue(ccl_tiles, dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(g.batch)), kThreads, 0, s, 
       g, mask, bits, labels, run, tile_rows, tile_cols);
-  EDAB_LAUNCH("ccl_tiles");
   // the edges between tiles
   for_voxels(s, g, [=] __device__(int64_t b) { return run == nullptr || run[b] != 0; },
              [=] __device__(int64_t b, int64_t v, int64_t i) {

@@ -134,3 +134,32 @@ def test_the_product_of_the_transforms_changed_during_calls(lib):
                 check(lib, x)
     finally:
         eda.set_transform_precision("tf32x3")
+
+
+def test_another_thread_synchronises_the_device(lib):
+    """The sequences are built without a capture, during which no thread may synchronise the device."""
+    import torch
+
+    torch.cuda.synchronize()
+    ends, errors, rounds = threading.Event(), [], [0]
+
+    def synchronise():
+        while not ends.is_set():
+            try:
+                torch.cuda.synchronize()
+                rounds[0] += 1
+            except RuntimeError as e:
+                errors.append(str(e))
+                return
+
+    t = threading.Thread(target=synchronise)
+    t.start()
+    try:
+        for i in range(8):
+            for shape in ((1, 900 + 2 * i), (1, 24 + i, 33)):
+                for seed in range(4):
+                    check(lib, field(shape, np.float32, seed))
+    finally:
+        ends.set()
+        t.join()
+    assert rounds[0] > 0 and not errors
