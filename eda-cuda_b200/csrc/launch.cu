@@ -9,6 +9,8 @@ thread_local Sequence* t_building = nullptr;
 
 }  // namespace
 
+bool building_sequence() { return t_building != nullptr; }
+
 Sequence::Sequence() {
   EDAB_CUDA(cudaGraphCreate(&graph_, 0));
   t_building = this;

@@ -28,6 +28,7 @@ class Sequence {
   cudaGraphNode_t last_ = nullptr;
 };
 
+bool building_sequence();  // by the calling thread
 void enqueue_config(const cudaLaunchConfig_t& at, const void* kernel, void** args);
 
 // kernel<<<grid, block, smem, s>>>(args...) with clusters of cluster_x CTAs, counted and checked; into

@@ -38,7 +38,8 @@ void once_on_device(const void* key, const std::function<void()>& set) {
   seen.emplace(dev, key);
 }
 
-bool profiling() { return g_on.load(std::memory_order_relaxed); }
+// (never into a sequence that is being built: it would count on every replay, whether on or off)
+bool profiling() { return g_on.load(std::memory_order_relaxed) && !building_sequence(); }
 
 unsigned long long* cube_bytes_counter() {
   if (!profiling()) return nullptr;

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -163,3 +164,35 @@ def test_another_thread_synchronises_the_device(lib):
         ends.set()
         t.join()
     assert rounds[0] > 0 and not errors
+
+
+def counts(lib):
+    n, passes, moved, ms = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_double(), ctypes.c_double()
+    assert lib.eda_profile_read(ctypes.byref(n), ctypes.byref(passes), ctypes.byref(moved), ctypes.byref(ms)) == 0
+    return n.value, passes.value, moved.value
+
+
+def test_instrumentation_switched_during_calls(lib):
+    """Sequences hold no instrumentation: with it off again, replays count no bytes and no passes."""
+    ends = threading.Event()
+
+    def switch():
+        while not ends.is_set():
+            lib.eda_profile(1)
+            time.sleep(1e-3)
+            lib.eda_profile(0)
+            time.sleep(1e-3)
+
+    xs = [field((1, 1300 + 2 * i), np.float32, i) for i in range(6)]
+    t = threading.Thread(target=switch)
+    t.start()
+    for x in xs[::-1]:
+        for _ in range(6):
+            results(x)
+    ends.set()
+    t.join()
+    for x in xs:
+        lib.eda_profile(0)
+        results(x)
+        assert counts(lib)[1:] == (0, 0.0)
+        check(lib, x)
