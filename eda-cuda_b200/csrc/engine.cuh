@@ -46,7 +46,7 @@ void cuda_fail(cudaError_t e, const char* what, const char* file, int line);
   } while (0)
 // Every kernel launch is counted for the instrumentation (profile.cu) and checked: by enqueue (launch.hpp:
 // the engine's steps), or by EDAB_LAUNCH after it.
-void note_launch();
+void note_launch(int64_t launches = 1);
 // Runs set(), which sets attributes of kernel `key` on the current device (such as its dynamic
 // shared-memory limit: they are per device), on the first call for that kernel and device. Every
 // other call, from any host thread, returns only once set() has completed, so no launch can

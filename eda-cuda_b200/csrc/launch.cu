@@ -32,6 +32,7 @@ void Sequence::kernel(const cudaLaunchConfig_t& at, const void* f, void** args) 
   EDAB_CUDA(cudaGraphAddKernelNode(&node, graph_, after(), last_ ? 1 : 0, &p));
   for (unsigned i = 0; i < at.numAttrs; ++i) EDAB_CUDA(cudaGraphKernelNodeSetAttribute(node, at.attrs[i].id, &at.attrs[i].val));
   last_ = node;
+  ++launches_;
 }
 
 void Sequence::zero(void* p, size_t bytes) {

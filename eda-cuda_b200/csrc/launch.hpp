@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <cstdint>
 #include <tuple>
 
 namespace edab {
@@ -21,11 +22,13 @@ class Sequence {
   void kernel(const cudaLaunchConfig_t& at, const void* f, void** args);
   void zero(void* p, size_t bytes);
   cudaGraphExec_t instantiate();
+  int64_t launches() const { return launches_; }  // its kernels
 
  private:
   cudaGraphNode_t* after() { return last_ ? &last_ : nullptr; }
   cudaGraph_t graph_ = nullptr;
   cudaGraphNode_t last_ = nullptr;
+  int64_t launches_ = 0;
 };
 
 bool building_sequence();  // by the calling thread

@@ -25,7 +25,7 @@ __device__ unsigned long long g_cube_bytes;
 
 }  // namespace
 
-void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+void note_launch(int64_t launches) { g_launches.fetch_add(launches, std::memory_order_relaxed); }
 
 void once_on_device(const void* key, const std::function<void()>& set) {
   static std::mutex mu;

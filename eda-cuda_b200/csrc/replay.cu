@@ -38,6 +38,7 @@ void Replays::run(const std::string& key, cudaStream_t s, const std::function<vo
       Sequence q;
       issue();
       e.exec = q.instantiate();
+      e.launches = q.launches();
     } catch (const std::exception&) {
       // the sequence is issued directly, where an error that is its own shows
     }
@@ -46,8 +47,12 @@ void Replays::run(const std::string& key, cudaStream_t s, const std::function<vo
       (void)cudaGetLastError();
     }
   }
-  if (e.exec) EDAB_CUDA(cudaGraphLaunch(e.exec, s));
-  else issue();
+  if (!e.exec) {
+    issue();
+    return;
+  }
+  EDAB_CUDA(cudaGraphLaunch(e.exec, s));
+  note_launch(e.launches);
 }
 
 }  // namespace edab

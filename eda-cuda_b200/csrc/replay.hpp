@@ -29,6 +29,7 @@ class Replays {
     cudaGraphExec_t exec = nullptr;
     bool refused = false;  // could not be built: always issued directly
     uint64_t used = 0;
+    int64_t launches = 0;  // of the graph
   };
   // The least recently used sequence leaves beyond this many: a program that cycles through more never
   // comes to its second use, so it builds no graph.

@@ -196,3 +196,15 @@ def test_instrumentation_switched_during_calls(lib):
         results(x)
         assert counts(lib)[1:] == (0, 0.0)
         check(lib, x)
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=["x".join(map(str, s)) for s in SHAPES])
+def test_replayed_launches_are_counted(lib, shape):
+    x = field(shape, np.float32, 5)
+    launches = []
+    for on in (1, 0, 0, 0):
+        lib.eda_profile(on)
+        results(x)
+        launches.append(counts(lib)[0])
+    lib.eda_profile(0)
+    assert launches[0] > 20 and len(set(launches)) == 1, launches
