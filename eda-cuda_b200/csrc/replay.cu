@@ -4,7 +4,14 @@
 
 #include "engine.cuh"
 
+#include <atomic>
+
 namespace edab {
+namespace {
+std::atomic<int64_t> g_built{0}, g_launched{0}, g_refused{0}, g_evicted{0};
+}
+
+ReplayCounts replay_counts() { return {g_built, g_launched, g_refused, g_evicted}; }
 
 void Replays::clear() {
   for (auto& [key, e] : entries_) {
@@ -24,6 +31,7 @@ void Replays::run(const std::string& key, cudaStream_t s, const std::function<vo
       if (old->second.exec) {
         EDAB_CUDA(cudaStreamSynchronize(s));  // its last launch may still run
         cudaGraphExecDestroy(old->second.exec);
+        ++g_evicted;
       }
       entries_.erase(old);
     }
@@ -39,11 +47,13 @@ void Replays::run(const std::string& key, cudaStream_t s, const std::function<vo
       issue();
       e.exec = q.instantiate();
       e.launches = q.launches();
+      ++g_built;
     } catch (const std::exception&) {
       // the sequence is issued directly, where an error that is its own shows
     }
     if (!e.exec) {
       e.refused = true;
+      ++g_refused;
       (void)cudaGetLastError();
     }
   }
@@ -53,6 +63,7 @@ void Replays::run(const std::string& key, cudaStream_t s, const std::function<vo
   }
   EDAB_CUDA(cudaGraphLaunch(e.exec, s));
   note_launch(e.launches);
+  ++g_launched;
 }
 
 }  // namespace edab

@@ -16,6 +16,13 @@
 
 namespace edab {
 
+// What the process's sequences came to: graphs built and launched, sequences that could not be built, and
+// graphs that left for others (the tests' evidence that calls replay).
+struct ReplayCounts {
+  int64_t built, launched, refused, evicted;
+};
+ReplayCounts replay_counts();
+
 class Replays {
  public:
   ~Replays() { clear(); }

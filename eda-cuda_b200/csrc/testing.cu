@@ -345,3 +345,14 @@ extern "C" int eda_testing_components(const uint8_t* mask_dev, int bits, int dim
     run_components(mask_dev, bits, dim, batch, n, labels_dev, static_cast<cudaStream_t>(stream));
   });
 }
+
+extern "C" int eda_testing_replays(int64_t* built, int64_t* launched, int64_t* refused, int64_t* evicted) {
+  return guarded("eda_testing_replays", [&] {
+    if (!built || !launched || !refused || !evicted) throw std::invalid_argument("eda_testing_replays: null argument");
+    const ReplayCounts c = replay_counts();
+    *built = c.built;
+    *launched = c.launched;
+    *refused = c.refused;
+    *evicted = c.evicted;
+  });
+}

@@ -63,6 +63,11 @@ EDA_API int eda_testing_flags(const void* r_dev, const void* tau_dev, int dtype,
 EDA_API int eda_testing_components(const uint8_t* mask_dev, int bits, int dim, int64_t batch, const int64_t* n,
                                    int32_t* labels_dev, void* stream);
 
+/* What the replayed launch sequences of the process came to so far: graphs built, launches of them,
+ * sequences that could not be built, and graphs that left their cache for others. No counterpart in the
+ * reference, which issues every launch. */
+EDA_API int eda_testing_replays(int64_t* built, int64_t* launched, int64_t* refused, int64_t* evicted);
+
 #ifdef __cplusplus
 }
 #endif

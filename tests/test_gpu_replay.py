@@ -60,9 +60,17 @@ def check(lib, x, **kw):
 SHAPES = [(1, 2048), (3, 300), (2, 41, 67), (3, 9, 14, 33), (1, 2), (70, 513), (1, 20011)]
 
 
+def replays(lib):
+    """Graphs built, launches of them, sequences refused, graphs evicted so far."""
+    out = [ctypes.c_int64() for _ in range(4)]
+    assert lib.eda_testing_replays(*(ctypes.byref(c) for c in out)) == 0
+    return np.array([c.value for c in out])
+
+
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("shape", SHAPES, ids=["x".join(map(str, s)) for s in SHAPES])
 def test_calls_of_one_geometry(lib, shape, dtype):
+    before = replays(lib)
     for seed in range(4):
         x = field(shape, dtype, seed)
         if seed == 1:
@@ -70,19 +78,31 @@ def test_calls_of_one_geometry(lib, shape, dtype):
         if seed == 2:
             x[0].reshape(-1)[1] = np.nan  # one that fails
         check(lib, x)
+    built, launched, refused, _ = replays(lib) - before
+    assert built > 0 and launched >= built and refused == 0
 
 
 def test_geometries_and_constants_in_turn(lib):
+    for shape in SHAPES:  # (the first graphs, which the others push out)
+        for seed in range(3):
+            check(lib, field(shape, np.float32, seed))
+    before = replays(lib)
     for seed in range(2):
         for shape in SHAPES:  # (each has several sequences: more than the cache keeps)
             for kw in ({}, {"max_imf": 2}, {"tie_tolerance": 0.01}, {"check_finite": False}):
                 check(lib, field(shape, np.float32, seed), **kw)
+    _, _, refused, evicted = replays(lib) - before
+    assert evicted > 0 and refused == 0
 
 
 @pytest.mark.parametrize("shape", [(4, 512, 512), (5, 512, 512)], ids=["at the limit", "above"])
 def test_size_rule(lib, shape):
-    for seed in range(2):
+    before = replays(lib)
+    for seed in range(3):
         check(lib, field(shape, np.float32, seed), max_imf=2)
+    built, launched, refused, _ = replays(lib) - before
+    assert refused == 0
+    assert (built > 0 and launched > 0) if shape[0] == 4 else (built == 0 and launched == 0)
 
 
 def test_streams_and_threads(lib):
