@@ -588,6 +588,7 @@ std::unique_ptr<Run> decompose_impl(const void* x, bool on_device, const SourceV
   }
   run->chunk = Bc;
   ws.reserve(need(Bc), s);
+  if (Replays* r = ws.replays()) r->begin_call();
   std::vector<Elem> elems(static_cast<size_t>(batch));
   std::vector<int32_t> exps(static_cast<size_t>(batch), 0);
   std::vector<Elem> part;

@@ -35,13 +35,15 @@ void Replays::run(const std::string& key, cudaStream_t s, const std::function<vo
       }
       entries_.erase(old);
     }
-    entries_[key].used = ++clock_;
+    Entry& e = entries_[key];
+    e.used = ++clock_;
+    e.first = call_;
     issue();
     return;
   }
   Entry& e = it->second;
   e.used = ++clock_;
-  if (!e.exec && !e.refused) {
+  if (!e.exec && !e.refused && e.first != call_) {
     try {
       Sequence q;
       issue();

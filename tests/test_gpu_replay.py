@@ -228,3 +228,13 @@ def test_replayed_launches_are_counted(lib, shape):
         launches.append(counts(lib)[0])
     lib.eda_profile(0)
     assert launches[0] > 20 and len(set(launches)) == 1, launches
+
+
+def test_sequences_are_built_in_a_second_call(lib):
+    """The modes of one call share their sequences: a geometry that is met once builds no graph."""
+    before = replays(lib)
+    for n in range(5000, 5040, 4):
+        results(field((1, n), np.float32, n))
+    assert not (replays(lib) - before)[:3].any()
+    results(field((1, 5036), np.float32, 5036))
+    assert (replays(lib) - before)[0] > 0
