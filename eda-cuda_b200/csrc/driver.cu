@@ -62,9 +62,7 @@ std::vector<std::unique_ptr<Workspace>>& idle_workspaces() {
 
 Workspace& thread_workspace() {
   thread_local Workspace ws;
-  if (t_leased) return *t_leased;
-  ws.keep_replays();
-  return ws;
+  return t_leased ? *t_leased : ws;
 }
 
 void set_thread_workspace(Workspace* ws) { t_leased = ws; }
@@ -588,7 +586,8 @@ std::unique_ptr<Run> decompose_impl(const void* x, bool on_device, const SourceV
   }
   run->chunk = Bc;
   ws.reserve(need(Bc), s);
-  if (Replays* r = ws.replays()) r->begin_call();
+  Replays* replays = p.replay ? &ws.replays() : nullptr;
+  if (replays) replays->begin_call();
   std::vector<Elem> elems(static_cast<size_t>(batch));
   std::vector<int32_t> exps(static_cast<size_t>(batch), 0);
   std::vector<Elem> part;
@@ -618,11 +617,11 @@ std::unique_ptr<Run> decompose_impl(const void* x, bool on_device, const SourceV
                         : nullptr;
     if (f32) {
       run_chunk<float>(gc, c, s, ws, static_cast<const float*>(staged), reinterpret_cast<float*>(rows0), hist_i + ho,
-                       hist_i + he + ho, hist_d + ho, hist_d + he + ho, part, reinterpret_cast<float*>(orient0));
+                       hist_i + he + ho, hist_d + ho, hist_d + he + ho, part, reinterpret_cast<float*>(orient0), replays);
     } else {
       run_chunk<double>(gc, c, s, ws, static_cast<const double*>(staged), reinterpret_cast<double*>(rows0),
                         hist_i + ho, hist_i + he + ho, hist_d + ho, hist_d + he + ho, part,
-                        reinterpret_cast<double*>(orient0));
+                        reinterpret_cast<double*>(orient0), replays);
     }
     for (int64_t b = 0; b < nb; ++b) elems[static_cast<size_t>(b0 + b)] = part[static_cast<size_t>(b)];
   }

@@ -34,16 +34,11 @@ class Workspace {
     return p;
   }
   void release();
-  // The launch sequences replayed on this buffer, for a workspace that lives as long as its thread
-  // (nullptr: a view of the caller's memory, or a workspace that ragged batches' workers lease, which
-  // meets other shapes on every call).
-  Replays* replays() { return keeps_replays_ ? &replays_ : nullptr; }
-  void keep_replays() { keeps_replays_ = true; }
+  Replays& replays() { return replays_; }  // the launch sequences replayed on this buffer
   const void* base() const { return base_; }
 
  private:
   Replays replays_;
-  bool keeps_replays_ = false;
   unsigned char* base_ = nullptr;
   size_t size_ = 0;
   size_t used_ = 0;
@@ -89,6 +84,8 @@ struct Params {
   int64_t max_chunk = 0;
   int64_t mem_budget = 0;  // > 0: the device bytes this call may hold (else the free memory)
   bool orientation = false;  // keep n and c of every mode (D >= 2): return_orientation
+  bool replay = true;        // calls of one geometry replay their launches (the groups of a ragged batch do not:
+                             // they meet other shapes on every call)
 };
 
 // One call's results: the rows (B, cap, count) on the device and the per-element information.
@@ -189,6 +186,7 @@ template <class T>
 size_t engine_bytes(const Geom& g);
 template <class T>
 void run_chunk(const Geom& g, const Ctl& c, cudaStream_t s, Workspace& ws, const T* x, T* rows, int32_t* hs,
-               int32_t* hf, double* hp, double* he, std::vector<Elem>& out, T* orient = nullptr);
+               int32_t* hf, double* hp, double* he, std::vector<Elem>& out, T* orient = nullptr,
+               Replays* replays = nullptr);
 
 }  // namespace edab

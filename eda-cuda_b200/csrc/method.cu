@@ -1741,7 +1741,7 @@ struct LongLineScratch {
 
 template <class T>
 void run_chunk(const Geom& g, const Ctl& c, cudaStream_t s, Workspace& ws, const T* x, T* rows, int32_t* hs,
-               int32_t* hf, double* hp, double* he, std::vector<Elem>& out, T* orient) {
+               int32_t* hf, double* hp, double* he, std::vector<Elem>& out, T* orient, Replays* replays) {
   Engine<T> e(g, c, s, ws);
   e.orient_out_ = g.dim >= 2 ? orient : nullptr;
   // replayed launches: for calls that the launches bound (up to 1 M samples: 4 float64 images of
@@ -1750,7 +1750,7 @@ void run_chunk(const Geom& g, const Ctl& c, cudaStream_t s, Workspace& ws, const
   // not for batches of uneven lengths (their lengths lie elsewhere on every call), nor while launches
   // are counted
   if (!g.len && g.batch * g.field <= (int64_t{1} << 20) && !profiling()) {
-    e.replays_ = ws.replays();
+    e.replays_ = replays;
     e.base_ = ws.base();
   }
   const size_t lb = long_line_scratch_bytes(g, sizeof(T));
@@ -1763,8 +1763,8 @@ void run_chunk(const Geom& g, const Ctl& c, cudaStream_t s, Workspace& ws, const
 template size_t engine_bytes<float>(const Geom&);
 template size_t engine_bytes<double>(const Geom&);
 template void run_chunk<float>(const Geom&, const Ctl&, cudaStream_t, Workspace&, const float*, float*, int32_t*,
-                               int32_t*, double*, double*, std::vector<Elem>&, float*);
+                               int32_t*, double*, double*, std::vector<Elem>&, float*, Replays*);
 template void run_chunk<double>(const Geom&, const Ctl&, cudaStream_t, Workspace&, const double*, double*,
-                                int32_t*, int32_t*, double*, double*, std::vector<Elem>&, double*);
+                                int32_t*, int32_t*, double*, double*, std::vector<Elem>&, double*, Replays*);
 
 }  // namespace edab

@@ -169,6 +169,7 @@ std::unique_ptr<RaggedRun> decompose_ragged(const void* const* xs, bool on_devic
   size_t free_b = 0, total_b = 0;
   EDAB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   Params pw = p;
+  pw.replay = false;
   if (nw > 1) pw.mem_budget = static_cast<int64_t>(free_b / static_cast<size_t>(nw));
   // the workers' streams start after the work the caller queued on s (the inputs' producers)
   cudaEvent_t ready = nullptr;
@@ -194,7 +195,7 @@ std::unique_ptr<RaggedRun> decompose_ragged(const void* const* xs, bool on_devic
         if (k >= order.size()) break;
         const int32_t gi = order[k];
         res->groups[static_cast<size_t>(gi)] = run_group(groups[static_cast<size_t>(gi)], xs, on_device, dtype, dim,
-                                                         nw > 1 ? pw : p, ws);
+                                                         pw, ws);
       }
     } catch (...) {
       std::lock_guard<std::mutex> lock(err_mu);

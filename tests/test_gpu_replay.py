@@ -238,3 +238,18 @@ def test_sequences_are_built_in_a_second_call(lib):
     assert not (replays(lib) - before)[:3].any()
     results(field((1, 5036), np.float32, 5036))
     assert (replays(lib) - before)[0] > 0
+
+
+@pytest.mark.parametrize("workers", [1, 4])
+def test_ragged_batches_issue_every_launch(lib, workers):
+    import eda
+
+    rng = np.random.default_rng(workers)
+    batches = [[rng.standard_normal(600).astype(np.float32) for _ in range(3)],  # one group of one length
+               [rng.standard_normal((20 + k, 30)).astype(np.float32) for k in range(3)],
+               [rng.standard_normal(s).astype(np.float32) for s in (100, 90, 2000, 2100, 77)]]
+    before = replays(lib)
+    for _ in range(3):
+        for xs in batches:
+            eda.decompose_ragged(xs, workers=workers)
+    assert not (replays(lib) - before).any()
