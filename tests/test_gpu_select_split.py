@@ -1,10 +1,12 @@
 # SPDX-License-Identifier: Apache-2.0
-"""The split form of the exact selections (stats.cu: large elements of large calls), bit for bit
+"""The split form of the exact selections (stats.cu: large elements in batches of 16 or more), bit for bit
 against the oracle: brackets that hold the ranks, ties that fill the list (handed on to the other
-forms), one value everywhere, ranks at both ends, masks, differences and centres, rows with padding,
-elements that do not run beside ones that do; both sides of the size rule."""
+forms), one value everywhere, ranks at both ends, masks, differences and centres, rows with padding;
+both sides of the size rule, and the launches of each."""
 
 from __future__ import annotations
+
+import ctypes
 
 import numpy as np
 import pytest
@@ -14,8 +16,10 @@ from test_gpu_stats import dev, gpu_select, items  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
-# 2^21 items in all and 65 536 per element are the split's; the first shape lies just below
-SHAPES = [(31, 256, 256), (9, 500, 523), (33, 65535), (3, 97, 88, 101), (40, 300, 311)]
+# 16 elements, 65 536 padded items each and 2^21 in all are the split's; three shapes lie just below
+SPLIT = [(32, 256, 256), (17, 500, 523), (33, 65535), (16, 97, 88, 101), (40, 300, 311)]
+BELOW = [(31, 256, 256), (15, 500, 523), (40, 256, 223)]
+SHAPES = SPLIT + BELOW
 
 
 def fields(shape, dtype, kind, seed):
@@ -47,7 +51,7 @@ def test_split_samples(dev, shape, dtype, kind):  # noqa: F811
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
-@pytest.mark.parametrize("shape", [(9, 500, 523), (3, 97, 88, 101)], ids=["2d", "3d"])
+@pytest.mark.parametrize("shape", [(17, 500, 523), (16, 97, 88, 101)], ids=["2d", "3d"])
 def test_split_masks_differences_and_centres(dev, shape, dtype):  # noqa: F811
     rng = np.random.default_rng(2)
     x = fields(shape, dtype, "normal", 9)
@@ -70,3 +74,22 @@ def test_split_masks_differences_and_centres(dev, shape, dtype):  # noqa: F811
                 v = items(x[b], 1, axes, None, 0, None if c is None else c[b])
                 assert out[b] == oracle.select(v), (axes, b)
                 assert cnt[b] == v.size
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_size_rule(dev, dtype):  # noqa: F811
+    """The split form's three launches come before those of the other forms."""
+    _, lib = dev
+    n, rest = ctypes.c_int64(), (ctypes.c_int64(), ctypes.c_double(), ctypes.c_double())
+
+    def launches(shape, **kw):
+        x = fields(shape, dtype, "normal", 1)
+        lib.eda_profile(0)
+        gpu_select(dev, x, **kw)
+        lib.eda_profile_read(ctypes.byref(n), *(ctypes.byref(v) for v in rest))
+        return n.value
+
+    for kw in ({}, {"src": 1, "axes": 3}):
+        assert launches((16, 500, 523), **kw) - launches((15, 500, 523), **kw) == 3
+        assert launches((32, 256, 256), **kw) - launches((31, 256, 256), **kw) == (3 if not kw else 0)
+    assert launches((40, 256, 256)) - launches((40, 255, 256)) == 3
