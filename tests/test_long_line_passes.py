@@ -2,7 +2,8 @@
 """The index arithmetic of the tiled long-line passes (cube_long.cu), restated on the CPU: a max / min
 tile covers every output's window with the block suffixes, prefixes and runs of blocks that it holds;
 a box tile finds every output's segment, chunk and carry in the parts of the line that it stages, and
-its buffers hold them, for short segments (folded in the tile) and long ones (carries from the table)."""
+its buffers hold them, for short segments (folded in the tile) and long ones (carries from the table);
+the table holds the chunks of every window."""
 
 from __future__ import annotations
 
@@ -121,3 +122,16 @@ def test_box_tiles_hold_their_segments(tile):
                     for c in range(m >> 5):
                         a, b = held[(k, c)]
                         assert (a, b) == (first + (k0 + k) * wa + 32 * c, a + 31)
+
+
+def test_windows_of_several_chunks_fit_the_table_of_totals():
+    """The chunk totals of a window's segments (nseg cps, when a segment has more than one chunk) fit the
+    tot_slots(n) = n / 8 + 24 that the box passes and the long lines' carries hold per line and direction."""
+    rng = random.Random(11)
+    for _ in range(200000):
+        n = rng.randint(2, 65536)
+        r = min(rng.randint(0, rng.choice([20, 200, 5000, 70000])), n - 1)
+        wa, cps = 2 * r + 1, (2 * r + 1 + 31) >> 5
+        o = ((n >> 1) + (n & 1) * (r + 1)) % wa
+        nseg = (n - 1 + r - o) // wa - (r - o) // wa + 1
+        assert cps == 1 or nseg * cps <= n // 8 + 24, (n, r, nseg, cps)
