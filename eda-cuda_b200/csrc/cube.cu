@@ -78,12 +78,6 @@ int lines_per_cta(const Geom& g, int axis, size_t es, size_t cap, size_t (*bytes
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// A first pass stages its input once for every rung of the ladder and both fields of a max + min
-// cube when the line groups alone fill the GPU; else every rung and field is a CTA of its own (one line
-// of 2048 samples, 7 rungs, max + min: 4.7 us against 64.8 us in one CTA; 64 lines of 4096: 17 against
-// 75 us; at 64 fields of 512 x 512 one staging for all is the faster: 293 against 7 x 66 us).
-constexpr int64_t kFillCtas = 148 * kCubeCtas;
-
 template <class T>
 void launch_pass(cudaStream_t s, const Geom& g, PassArgs<T> a) {
   const DevFacts f = dev_facts();
@@ -121,11 +115,16 @@ void launch_pass(cudaStream_t s, const Geom& g, PassArgs<T> a) {
     groups = outer * (g.stride[a.axis] / P);
   }
   const int nf = a.op == static_cast<int>(CubeOp::kMaxMin) ? 2 : 1;
+  // A first pass stages its input once for every rung of the ladder and both fields of a max + min
+  // cube when the line groups alone fill the GPU; else every rung and field is a CTA of its own (one line
+  // of 2048 samples, 7 rungs, max + min: 4.7 us against 64.8 us in one CTA; 64 lines of 4096: 17 against
+  // 75 us; at 64 fields of 512 x 512 one staging for all is the faster: 293 against 7 x 66 us).
+  const bool fills = groups * g.batch >= int64_t{kCubeCtas} * f.sms;
   // (an output over the input is only written by a CTA that has staged every line it reads and is
   // their only reader)
   const bool shared = a.in_stride == 0 && a.in1 == nullptr;
   const bool in_place = a.in0 != nullptr && (a.in0 == a.out0 || a.in0 == a.out1);
-  const bool together = shared && (in_place || groups * g.batch >= kFillCtas) && bytes(n, P, rows, sizeof(T)) <= f.smem;
+  const bool together = shared && (in_place || fills) && bytes(n, P, rows, sizeof(T)) <= f.smem;
   a.zr = together ? a.rungs : 1;
   a.zf = together ? nf : 1;
   if (groups > 0x7fffffffLL || g.batch > 65535) throw std::invalid_argument("edab: cube launch too large");

@@ -19,10 +19,6 @@ constexpr int kWarps = kCubeThreads / 32;
 // offset, k_lo the first segment, nseg their number, cps the 32-sample chunks of a segment.
 struct Win {
   int32_t r, wa, o, k_lo, nseg, cps;
-  // the segments a CTA folds, relative to k_lo: segments [hk0, hk0 + hn) of the reversed line for
-  // H and [gk0, gk0 + gn) of the line for G (a whole line: 0 and nseg both; a tile of a long line:
-  // the segments its outputs need)
-  int32_t hk0, hn, gk0, gn;
 };
 // 32-bit arithmetic (the 64-bit integer divisions of a general formula are long emulated sequences
 // on the GPU): n (wa + 1) / 2 = n (r + 1) modulo wa = 2r + 1, where 2 (r + 1) = 1, is n / 2 for an
@@ -41,8 +37,6 @@ __device__ __forceinline__ Win make_win(int32_t n, int32_t w) {
   const int32_t k_hi = floor_div32(n - 1 + q.r - q.o, q.wa);
   q.nseg = k_hi - q.k_lo + 1;
   q.cps = (q.wa + 31) >> 5;
-  q.hk0 = q.gk0 = 0;
-  q.hn = q.gn = q.nseg;
   return q;
 }
 
@@ -59,6 +53,23 @@ __host__ __device__ constexpr int32_t row_stride(int32_t n) {
 template <class T>
 __host__ __device__ constexpr int32_t group_elems(int32_t n, int P, bool rows) {
   return rows ? P * row_stride<T>(n) : ((n * P + 3) & ~3);
+}
+
+// Order keys are signed integers of the samples' size.
+template <class T>
+struct KeyType;
+template <>
+struct KeyType<float> {
+  using type = int32_t;
+};
+template <>
+struct KeyType<double> {
+  using type = long long;
+};
+template <class K>
+__device__ __forceinline__ K key_min() {
+  if constexpr (sizeof(K) == 4) return INT_MIN;
+  else return LLONG_MIN;
 }
 
 // Order key of v as an integer: integer order = order of max_c / min_c; its own inverse on the bits.

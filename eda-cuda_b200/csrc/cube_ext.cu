@@ -29,25 +29,10 @@ namespace edab {
 namespace cubes {
 namespace {
 
-template <class T>
-struct KeyType;
-template <>
-struct KeyType<float> {
-  using type = int32_t;
-};
-template <>
-struct KeyType<double> {
-  using type = long long;
-};
 __device__ __forceinline__ int32_t bits_of(float v) { return __float_as_int(v); }
 __device__ __forceinline__ long long bits_of(double v) { return __double_as_longlong(v); }
 __device__ __forceinline__ float value_bits(int32_t k) { return __int_as_float(k); }
 __device__ __forceinline__ double value_bits(long long k) { return __longlong_as_double(k); }
-template <class K>
-__device__ __forceinline__ K key_min() {
-  if constexpr (sizeof(K) == 4) return INT_MIN;
-  else return LLONG_MIN;
-}
 
 // The longest blocks: short ones keep the CTA's threads busy on short lines (512 samples of 8 lines
 // are 256 blocks of 16 in rows for 256 threads), long ones keep the table small on long lines.

@@ -28,22 +28,6 @@ namespace edab {
 namespace cubes {
 namespace {
 
-template <class T>
-struct KeyType;
-template <>
-struct KeyType<float> {
-  using type = int32_t;
-};
-template <>
-struct KeyType<double> {
-  using type = long long;
-};
-template <class K>
-__device__ __forceinline__ K key_min() {
-  if constexpr (sizeof(K) == 4) return INT_MIN;
-  else return LLONG_MIN;
-}
-
 // The scratch: the lines' samples or keys [B][pitch] and per field (max; min as the complements' max)
 // the blocks' extremes [2][B][pitch / 32]; apart from them the chunk totals [rungs][B][2][TSL] and the
 // counts of the totals' CTAs that are done [rungs][B].

@@ -275,8 +275,8 @@ __global__ void orient_collect_kernel(int64_t B, int32_t D, int64_t count, int32
 
 // The longest axis. 2-D and 3-D: the reference's limits (8192 float32, 4096 float64 samples; the
 // passes stage whole lines in shared memory). 1-D signals: up to kMaxLine1D samples in either
-// dtype (the reference stops at the 2-D limits); lines beyond the staged capacity fold in global
-// memory (cube.cu, stats.cu).
+// dtype (the reference stops at the 2-D limits); lines beyond the staged capacity are cut into
+// tiles (cube_long.cu, stats.cu).
 constexpr int32_t kMaxLine1D = 65536;
 int32_t max_axis(int dtype, int dim) { return dim == 1 ? kMaxLine1D : (dtype == 0 ? 8192 : 4096); }
 

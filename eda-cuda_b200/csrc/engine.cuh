@@ -432,8 +432,8 @@ void cube_tune_override(const CubeTune* t);  // nullptr: none (per calling threa
 size_t long_line_scratch_bytes(const Geom& g, size_t es);
 size_t long_totals_scratch_bytes(const Geom& g, size_t es);
 void set_long_line_scratch(void* lines, void* totals);
-// What a call with 1-D lines of more than a CTA's shared memory (18 900 float32 samples) is accounted
-// for besides the engine's fields (engine_bytes).
+// What a call with 1-D lines of more than a CTA's shared memory (17 696 float32 or 8832 float64 samples) is
+// accounted for besides the engine's fields (engine_bytes); nothing takes it.
 size_t fold_scratch_bytes(const Geom& g, size_t es);
 
 // Canonical reductions: per element sum v^2 (canonical tree) and max|v| of f.

@@ -1716,7 +1716,9 @@ void Engine<T>::run(const T* x, T* rows_out, int32_t* hist_scale, int32_t* hist_
 // What a call of this geometry is accounted for, in the device memory that the batch is chunked by and
 // in the fixed scratch of the calls that allocate nothing: 24 fields of a sift and, for the longest
 // 1-D lines, a fold scratch. A run takes less (18 fields; the long lines' scratch lies in the fields
-// left over, the chunk totals of their box passes in the rungs' minima, which no box pass holds).
+// left over, the chunk totals of their box passes in the rungs' minima, which no box pass holds). The
+// accounting stays at what earlier passes took because it is a limit that callers see: which calls fit
+// the fixed scratch, how a batch is chunked under a budget (5 % of a 2-D call's workspace is not touched).
 template <class T>
 size_t engine_bytes(const Geom& g) {
   const size_t F = static_cast<size_t>(g.batch * g.field);

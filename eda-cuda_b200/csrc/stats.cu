@@ -1313,10 +1313,6 @@ void select(cudaStream_t s, const Geom& g, const Sel<T>& sel, double q, const in
     a.items = static_cast<int64_t>(a.naxes) * g.field;
   }
   if (g.batch > 65535) throw std::invalid_argument("edab: select batch too large");
-  // Otherwise clusters (one launch): of 256-thread CTAs when the batch fills the GPU with them, else of
-  // 1024-thread CTAs while an element has at most 8 items for each of their threads; larger elements of
-  // small batches take the grid-wide form, a launch per digit over many CTAs (133 000 items: 26 us for
-  // 32-bit keys, against 54 us in one cluster).
   int sms = 148;
   {
     int dev = 0;
@@ -1356,6 +1352,10 @@ void select(cudaStream_t s, const Geom& g, const Sel<T>& sel, double q, const in
     go(select_small<T, uint64_t>);
     return;
   }
+  // Otherwise clusters (one launch): of 256-thread CTAs when the batch fills the GPU with them, else of
+  // 1024-thread CTAs while an element has at most 8 items for each of their threads; larger elements of
+  // small batches take the grid-wide form, a launch per digit over many CTAs (133 000 items: 26 us for
+  // 32-bit keys, against 54 us in one cluster).
   const bool many = g.batch * kSelClusterMax >= 2 * static_cast<int64_t>(sms);
   if (!kSelClusters || (!many && a.items > int64_t{kSelClusterMax} * kSelWide * 8)) {
     if (!scratch) throw std::logic_error("edab: the grid-wide selection needs its scratch");

@@ -129,7 +129,7 @@ def test_config_ragged_1d(engine):
 
 def test_config_long_1d_signals(engine):
     """Signals of the 1-D ragged recipe beyond the 8192 samples that a pass stages in shared memory,
-    up to the recipe's 65536: their lines fold in global memory."""
+    up to the recipe's 65536: their lines run in tiles."""
     xs = [x for x in bench.signals_ragged(40, 256, 65536, 77) if x.size > 8192][:3]
     xs.append(bench.signals_ragged(1, 65536, 65537, 5)[0])  # exp(U[ln 65536, ln 65537]) truncates to 65536
     assert all(x.size > 8192 for x in xs) and xs[-1].size == 65536

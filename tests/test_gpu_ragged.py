@@ -201,7 +201,7 @@ def test_length_class_across_the_staged_capacity(torch):
 
 
 def test_length_class_of_the_longest_signals(torch):
-    """The class [32768, 65536]: global-memory folds, the global-memory extrema pass (lines beyond
+    """The class [32768, 65536]: the long lines' tiles, the global-memory extrema pass (lines beyond
     the staged extrema capacity) and column tiles in the components."""
     import eda
 
