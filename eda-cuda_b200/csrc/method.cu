@@ -1749,8 +1749,8 @@ void run_chunk(const Geom& g, const Ctl& c, cudaStream_t s, Workspace& ws, const
   // replayed launches: for calls that the launches bound (up to 1 M samples: 4 float64 images of
   // 333 x 500 took 18.1 ms issued, 16.2 ms replayed and 14.3 ms of kernels when this was drawn, 16 float32
   // ones of 512 x 512 37 ms issued and 36 ms of kernels);
-  // not for batches of uneven lengths (their lengths lie elsewhere on every call), nor while launches
-  // are counted
+  // not for batches of uneven lengths (their lengths lie elsewhere on every call), nor while the cube passes
+  // are instrumented
   if (!g.len && g.batch * g.field <= (int64_t{1} << 20) && !profiling()) {
     e.replays_ = replays;
     e.base_ = ws.base();

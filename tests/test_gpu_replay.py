@@ -2,7 +2,8 @@
 """Replayed launch sequences (replay.hpp) give what the same launches issued one by one give, bit for
 bit: the first, second and later calls of a geometry, on other data each time; geometries in turn,
 more of them than the cache keeps; another constant of the call; fields that fail; other streams and
-threads; both sides of the size rule. Calls whose launches are counted (eda_profile) issue every one."""
+threads; both sides of the size rule; settings and instrumentation changed, and the device synchronised, by
+another thread meanwhile; the launches counted. Calls that are instrumented (eda_profile) issue every one."""
 
 from __future__ import annotations
 
